@@ -115,6 +115,7 @@ __global__ void __launch_bounds__(128) k_probe_intersect_queued(DeviceScene scen
 // all-opaque scene, each warp walking its own contiguous share with refills;
 // out[i] = 1 when visible, -1 when occluded (k_probe_shadow's encoding).
 struct ProbeShadowSource {
+    static constexpr bool FALLBACK = true;  // a target may be any triangle, with no leaf on record
     const DeviceScene& scene;
     const float3* org;
     const float3* dir;
@@ -139,7 +140,6 @@ struct ProbeShadowSource {
     __device__ __forceinline__ bool begin(uint32_t i, Ray& ray, AnyQuery& a) const {
         ray = make_ray(org[i], dir[i]);
         const uint32_t light = targets[i].x, leaf = leaf_of(i);
-        a.occluded = false;
         a.light = light;
         a.lprim = targets[i].y;
         a.tm = tmaxs[i];

@@ -25,7 +25,12 @@ namespace cn {
 constexpr int TRAVERSAL_STACK = TRAVERSAL_STACK_DEPTH;
 
 struct Ray {
-    float3 org, dir, idir;
+    float3 org, dir;
+    // 1 / dir for the node test, bounded so a component of (nearly) zero gives
+    // finite planes: such a ray stays inside or outside a slab for the whole
+    // scene either way. A plane constant that overflows all the same turns
+    // into NaN, which the min/max of the node test skip (the slab accepts).
+    float3 idir;
     int kx, ky, kz;
     float sx, sy, sz;
     uint32_t oct_inv;  // bit 2: dir.x >= 0, bit 1: dir.y >= 0, bit 0: dir.z >= 0
@@ -37,7 +42,7 @@ __device__ __forceinline__ Ray make_ray(float3 org, float3 dir) {
     Ray r;
     r.org = org;
     r.dir = dir;
-    r.idir = f3(__fdiv_rn(1.0f, dir.x), __fdiv_rn(1.0f, dir.y), __fdiv_rn(1.0f, dir.z));
+    const float3 inv = f3(__fdiv_rn(1.0f, dir.x), __fdiv_rn(1.0f, dir.y), __fdiv_rn(1.0f, dir.z));
     float ax = fabsf(dir.x), ay = fabsf(dir.y), az = fabsf(dir.z);
     int kz = (ax > ay) ? (ax > az ? 0 : 2) : (ay > az ? 1 : 2);
     int kx = kz + 1 == 3 ? 0 : kz + 1;
@@ -54,9 +59,11 @@ __device__ __forceinline__ Ray make_ray(float3 org, float3 dir) {
     // The shear constants (Woop et al. 2013) from the reciprocal already
     // taken: any per-ray constants keep the test watertight, as long as every
     // triangle of the ray uses the same ones.
-    r.sz = comp(r.idir, kz);
+    r.sz = comp(inv, kz);
     r.sx = __fmul_rn(comp(dir, kx), r.sz);
     r.sy = __fmul_rn(comp(dir, ky), r.sz);
+    const float lim = fabsf(r.sz) * 1e30f;
+    r.idir = f3(fminf(fmaxf(inv.x, -lim), lim), fminf(fmaxf(inv.y, -lim), lim), fminf(fmaxf(inv.z, -lim), lim));
     r.oct_inv = (dir.x >= 0.0f ? 4u : 0u) | (dir.y >= 0.0f ? 2u : 0u) | (dir.z >= 0.0f ? 1u : 0u);
     return r;
 }
@@ -93,12 +100,82 @@ __device__ __forceinline__ bool tri_hit(const Ray& r, float4 a, float4 b, float4
     return true;
 }
 
-__device__ __forceinline__ uint32_t byte_of(uint32_t lo4, uint32_t hi4, int i) {
-    return ((i < 4 ? lo4 : hi4) >> (8 * (i & 3))) & 0xffu;
+// ---- node test ------------------------------------------------------------------
+//
+// The node test is the walk's inner loop and was bound by its 48 byte-to-float
+// conversions per node: I2F runs on the XU at an eighth of the FMA rate, and
+// the XU measured 86 % busy in the test alone (453 SM cycles per warp and
+// node; a 57-60 % busy XU was the walks' largest single pipe). Here a byte
+// becomes a float by one dp4a on the FMA pipe: the byte times 128 lands on the
+// low mantissa bits of 65536.0f (whose unit in the last place is 2^-7), which
+// gives 65536 + byte exactly, and the 65536 folds into the plane's constant.
+// Near and far plane go through one packed FMA, and the slab limits through
+// three-operand min/max: 304 cycles. Measured beside it: a byte permute
+// instead of dp4a 366 (the permute shares the ALU pipe with min/max and the
+// compares), one axis by I2F 330, unpacked FMAs 335.
+
+constexpr float PLANE_BIAS = 65536.0f;
+
+#ifdef __CUDA_ARCH__
+__device__ __forceinline__ float biased_byte(uint32_t w, int i) {
+    return __uint_as_float(__dp4a(w, 0x80u << (8 * i), 0x47800000u));
+}
+__device__ __forceinline__ uint32_t byte_at(uint32_t w, int i) { return __dp4a(w, 1u << (8 * i), 0u); }
+__device__ __forceinline__ float max3f(float a, float b, float c) {
+    float d;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+__device__ __forceinline__ float min3f(float a, float b, float c) {
+    float d;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+// (n, f) = (a · s + cn, b · s + cf), each one rounding: one packed instruction.
+struct PlanePair {
+    unsigned long long s, c;
+};
+__device__ __forceinline__ unsigned long long pack2(float a, float b) {
+    unsigned long long d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+    return d;
+}
+__device__ __forceinline__ PlanePair plane_pair(float s, float cn, float cf) { return {pack2(s, s), pack2(cn, cf)}; }
+__device__ __forceinline__ void plane_t(float a, float b, const PlanePair& p, float& n, float& f) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(pack2(a, b)), "l"(p.s), "l"(p.c));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(n), "=f"(f) : "l"(d));
+}
+#else  // the host harness: the same values from portable operations
+inline float biased_byte(uint32_t w, int i) { return PLANE_BIAS + float((w >> (8 * i)) & 0xffu); }
+inline uint32_t byte_at(uint32_t w, int i) { return (w >> (8 * i)) & 0xffu; }
+inline float max3f(float a, float b, float c) { return fmaxf(fmaxf(a, b), c); }
+inline float min3f(float a, float b, float c) { return fminf(fminf(a, b), c); }
+struct PlanePair {
+    float s, cn, cf;
+};
+inline PlanePair plane_pair(float s, float cn, float cf) { return {s, cn, cf}; }
+inline void plane_t(float a, float b, const PlanePair& p, float& n, float& f) {
+    n = fmaf(a, p.s, p.cn);
+    f = fmaf(b, p.s, p.cf);
+}
+#endif
+
+// One axis of a node: the ray reaches the plane of byte q at parameter
+// (65536 + q) · aid + c with c = aor - 65536 · aid, aid the axis's cell over
+// the direction and aor the node's corner relative to the origin over it. All
+// its roundings (aor's two, c's, the FMA's) are within 2^-22 of
+// s = 65536 |aid| + |aor|, which bounds every plane's |t|; the near constant
+// is lowered by 2^-21 s and the far one raised by 2^-20 s, so the test also
+// accepts whatever the plain test q · aid + aor with its far planes scaled by
+// 1.0000004 accepts: a walk visits the same nodes and now and then one more,
+// and commits the same hits. The slack is below 0.07 of a cell.
+__device__ __forceinline__ PlanePair node_axis(float aid, float aor) {
+    const float s = fmaf(fabsf(aid), PLANE_BIAS, fabsf(aor));
+    const float c = fmaf(-PLANE_BIAS, aid, aor);
+    return plane_pair(aid, fmaf(-0x1p-21f, s, c), fmaf(0x1p-20f, s, c));
 }
 
-// Intersect the eight children of node `ni`. Returns the hit mask; fills the
-// node's child/triangle base indices and inner mask.
 __device__ __forceinline__ uint4 ld_shared4(uint32_t addr) {
     uint4 v;
 #ifdef __CUDA_ARCH__
@@ -122,7 +199,11 @@ __device__ __forceinline__ void stage_top_levels(DeviceScene& s, uint4* smem, ui
 #endif
 }
 
-__device__ __forceinline__ uint32_t intersect_node(const DeviceScene& s, uint32_t ni, const Ray& r, float tmax,
+// Intersect the eight children of node `ni`. Returns the hit mask; fills the
+// node's child/triangle base indices and inner mask. `R`: a ray with org,
+// idir and oct_inv.
+template <class R>
+__device__ __forceinline__ uint32_t intersect_node(const DeviceScene& s, uint32_t ni, const R& r, float tmax,
                                                    uint32_t& base_child, uint32_t& base_tri, uint32_t& imask) {
     uint4 n0, n1, n2, n3, n4;
     if (ni < s.top_count) {
@@ -147,8 +228,9 @@ __device__ __forceinline__ uint32_t intersect_node(const DeviceScene& s, uint32_
     imask = n0.w >> 24;
     base_child = n1.x;
     base_tri = n1.y;
-    float3 aid = f3(sx * r.idir.x, sy * r.idir.y, sz * r.idir.z);
-    float3 aor = f3((p.x - r.org.x) * r.idir.x, (p.y - r.org.y) * r.idir.y, (p.z - r.org.z) * r.idir.z);
+    const PlanePair px = node_axis(sx * r.idir.x, (p.x - r.org.x) * r.idir.x);
+    const PlanePair py = node_axis(sy * r.idir.y, (p.y - r.org.y) * r.idir.y);
+    const PlanePair pz = node_axis(sz * r.idir.z, (p.z - r.org.z) * r.idir.z);
     // Near/far plane words per axis, swapped for negative directions.
     uint32_t nx0 = n2.x, nx1 = n2.y, fx0 = n3.z, fx1 = n3.w;
     uint32_t ny0 = n2.z, ny1 = n2.w, fy0 = n4.x, fy1 = n4.y;
@@ -156,7 +238,7 @@ __device__ __forceinline__ uint32_t intersect_node(const DeviceScene& s, uint32_
     if (r.idir.x < 0.0f) { uint32_t t0 = nx0, t1 = nx1; nx0 = fx0; nx1 = fx1; fx0 = t0; fx1 = t1; }
     if (r.idir.y < 0.0f) { uint32_t t0 = ny0, t1 = ny1; ny0 = fy0; ny1 = fy1; fy0 = t0; fy1 = t1; }
     if (r.idir.z < 0.0f) { uint32_t t0 = nz0, t1 = nz1; nz0 = fz0; nz1 = fz1; fz0 = t0; fz1 = t1; }
-    const float tlimit = tmax * 1.00002f;  // cull only nodes clearly beyond the current hit
+    const float tlimit = tmax * 1.000021f;  // cull only nodes clearly beyond the current hit
     // An inner child's meta byte is 0b001_11sss (bit 24 + slot); XOR its slot
     // with the ray's octant for all eight children at once: bit 3 of a byte
     // is set where its bits 3 and 4 both are (inner children only: leaf
@@ -167,18 +249,16 @@ __device__ __forceinline__ uint32_t intersect_node(const DeviceScene& s, uint32_
     uint32_t mask = 0;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-        uint32_t meta = byte_of(ml, mh, i);  // 0 for an empty slot: contributes no bits
-        float tnx = fmaf(float(byte_of(nx0, nx1, i)), aid.x, aor.x);
-        float tny = fmaf(float(byte_of(ny0, ny1, i)), aid.y, aor.y);
-        float tnz = fmaf(float(byte_of(nz0, nz1, i)), aid.z, aor.z);
-        float tfx = fmaf(float(byte_of(fx0, fx1, i)), aid.x, aor.x);
-        float tfy = fmaf(float(byte_of(fy0, fy1, i)), aid.y, aor.y);
-        float tfz = fmaf(float(byte_of(fz0, fz1, i)), aid.z, aor.z);
-        float t0 = fmaxf(fmaxf(tnx, tny), fmaxf(tnz, 0.0f));
-        float t1 = fminf(fminf(tfx, tfy), fminf(tfz, tlimit)) * 1.0000004f;
-        if (t0 <= t1) {
-            mask |= (meta >> 5) << (meta & 0x1fu);
-        }
+        const int k = i & 3;
+        const bool lo = i < 4;
+        const uint32_t meta = byte_at(lo ? ml : mh, k);  // 0 for an empty slot: contributes no bits
+        float tnx, tny, tnz, tfx, tfy, tfz;
+        plane_t(biased_byte(lo ? nx0 : nx1, k), biased_byte(lo ? fx0 : fx1, k), px, tnx, tfx);
+        plane_t(biased_byte(lo ? ny0 : ny1, k), biased_byte(lo ? fy0 : fy1, k), py, tny, tfy);
+        plane_t(biased_byte(lo ? nz0 : nz1, k), biased_byte(lo ? fz0 : fz1, k), pz, tnz, tfz);
+        const float t0 = fmaxf(max3f(tnx, tny, tnz), 0.0f);
+        const float t1 = fminf(min3f(tfx, tfy, tfz), tlimit);
+        if (t0 <= t1) mask |= (meta >> 5) << (meta & 0x1fu);
     }
     return mask;
 }
@@ -225,8 +305,8 @@ __device__ __forceinline__ uint32_t walk_bound(const DeviceScene& s) { return 4u
 // have one), push what remains of the group and intersect the child: w.g
 // becomes its inner children, w.t its hit leaves' triangles. Returns false
 // when the stack is full.
-template <bool COUNT = false, int S = TRAVERSAL_STACK>
-__device__ __forceinline__ bool expand_node(const DeviceScene& s, const Ray& r, float tmax, Walk& w, uint2* stack,
+template <bool COUNT = false, int S = TRAVERSAL_STACK, class R>
+__device__ __forceinline__ bool expand_node(const DeviceScene& s, const R& r, float tmax, Walk& w, uint2* stack,
                                             uint32_t* visits) {
     uint32_t pos = 31u - __clz(w.g.y & 0xff000000u);
     w.g.y &= ~(1u << pos);

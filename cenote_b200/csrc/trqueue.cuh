@@ -39,34 +39,42 @@ constexpr uint32_t TQ_FULL = 0xffffffffu;
 // measured no gain from it).
 constexpr uint32_t TQ_WAITING = 8;
 
-// One warp's queue in shared memory (896 bytes), small enough that a full SM
-// of traversal blocks leaves the L1 cache (which holds the walks' stacks and
-// the nodes and triangles they revisit) almost all of its capacity.
+// One warp's queue in shared memory (1,792 bytes: a full SM of traversal
+// blocks keeps 56 KB, and the L1 cache, which holds the walks' stacks and the
+// nodes and triangles they revisit, most of its capacity). What a lane's ray
+// needs only in the triangle rounds lives here instead of in registers: ten
+// registers a lane, without which the node test spilled.
 struct TriQueueSmem {
     uint2 entry[TQ_CAP];     // (first triangle, owner lane << 24 | untested triangle bits)
-    // Per owner lane, a round's running minima of the candidates' t key and
-    // instance, then its primitive and the winning lane; ~0 between rounds.
+    // Per owner lane, a round's running minimum of the candidates' t key and
+    // the winning lane; ~0 between rounds. `key2` serves exact ties.
     uint32_t key[32], key2[32], winner[32];
+    // Per lane: the watertight test's shear constants (sx, sy, sz) and its
+    // axes kx | ky << 2 | kz << 4.
+    float4 shear[32];
+    // Per lane: the closest hit so far (instance, primitive, b1, b2), or a
+    // shadow query's target (leaf, instance, primitive, unused).
+    uint4 best[32];
 };
+
+// What a walking lane keeps of its ray: the node test's inputs.
+struct WalkRay {
+    float3 org, idir;
+    uint32_t oct_inv;
+};
+
+// Split a lane's ray between its registers and the warp's shared memory.
+__device__ __forceinline__ WalkRay tq_ray(TriQueueSmem& sm, const Ray& r) {
+    sm.shear[threadIdx.x & 31u] =
+        make_float4(r.sx, r.sy, r.sz, __uint_as_float(uint32_t(r.kx) | (uint32_t(r.ky) << 2) | (uint32_t(r.kz) << 4)));
+    return {r.org, r.idir, r.oct_inv};
+}
 
 // The warp's queue positions; every lane holds the same values. Entries
 // head .. tail-1 are pending; `tris` counts their untested bits.
 struct TriQueue {
     uint32_t head, tail, tris;
 };
-
-// The closest hit of a lane's ray so far.
-struct Closest {
-    float tmax, b1, b2;
-    uint32_t inst, prim;
-};
-
-__device__ __forceinline__ void closest_begin(Closest& c) {
-    c.tmax = 1e30f;
-    c.b1 = c.b2 = 0.0f;
-    c.inst = LIGHT_NONE;
-    c.prim = 0u;
-}
 
 // Position of the (k+1)-th lowest set bit of m (m has more than k set bits):
 // the largest x with popc(m below x) <= k, by binary search.
@@ -142,16 +150,17 @@ __device__ __forceinline__ TqWork tq_take(TriQueueSmem& sm, TriQueue& q) {
     return wk;
 }
 
-// The owner's ray as the watertight test reads it, over shuffles.
-__device__ __forceinline__ Ray owner_ray(const Ray& ray, uint32_t owner) {
+// The owner's ray as the watertight test reads it: its origin over shuffles,
+// the rest from shared memory.
+__device__ __forceinline__ Ray owner_ray(const TriQueueSmem& sm, const WalkRay& ray, uint32_t owner) {
     Ray ro;
     ro.org = f3(__shfl_sync(TQ_FULL, ray.org.x, owner), __shfl_sync(TQ_FULL, ray.org.y, owner),
                 __shfl_sync(TQ_FULL, ray.org.z, owner));
-    ro.sx = __shfl_sync(TQ_FULL, ray.sx, owner);
-    ro.sy = __shfl_sync(TQ_FULL, ray.sy, owner);
-    ro.sz = __shfl_sync(TQ_FULL, ray.sz, owner);
-    const uint32_t kp =
-        __shfl_sync(TQ_FULL, uint32_t(ray.kx) | (uint32_t(ray.ky) << 2) | (uint32_t(ray.kz) << 4), owner);
+    const float4 sh = sm.shear[owner];
+    ro.sx = sh.x;
+    ro.sy = sh.y;
+    ro.sz = sh.z;
+    const uint32_t kp = __float_as_uint(sh.w);
     ro.kx = int(kp & 3u);
     ro.ky = int((kp >> 2) & 3u);
     ro.kz = int((kp >> 4) & 3u);
@@ -162,13 +171,13 @@ __device__ __forceinline__ Ray owner_ray(const Ray& ray, uint32_t owner) {
 // ray; every owner commits the best of its candidates. All 32 lanes call it
 // together with q.tris > 0.
 template <bool COUNT = false>
-__device__ __forceinline__ void tq_round(const DeviceScene& s, TriQueueSmem& sm, TriQueue& q, const Ray& ray,
-                                         Closest& c, uint32_t ray_mask, uint32_t* tests) {
+__device__ __forceinline__ void tq_round(const DeviceScene& s, TriQueueSmem& sm, TriQueue& q, const WalkRay& ray,
+                                         float& tmax, uint32_t ray_mask, uint32_t* tests) {
     const uint32_t lane = threadIdx.x & 31u;
     const TqWork wk = tq_take(sm, q);
     const uint32_t owner = wk.owner;
-    const Ray ro = owner_ray(ray, owner);
-    const float tmo = __shfl_sync(TQ_FULL, c.tmax, owner);
+    const Ray ro = owner_ray(sm, ray, owner);
+    const float tmo = __shfl_sync(TQ_FULL, tmax, owner);
     bool cand = false;
     float t = 0.0f, b1 = 0.0f, b2 = 0.0f;
     uint32_t inst = 0u, prim = 0u;
@@ -182,41 +191,55 @@ __device__ __forceinline__ void tq_round(const DeviceScene& s, TriQueueSmem& sm,
             prim = __float_as_uint(b.w);
         }
     }
+    if (!__any_sync(TQ_FULL, cand)) {
+        __syncwarp();
+        return;
+    }
     // Per owner, the lexicographic minimum of (t, instance, primitive); both
     // zeros of t order as one, as they compare equal in the per-lane walk.
+    // The nearest t is a shared-memory minimum per owner (the slots start at
+    // ~0 and are reset by their owners after the round; grouping the lanes by
+    // owner with a warp match instead measured 30 % slower), and a lane alone
+    // at it wins. Only when two lanes of one owner meet at the same t do the
+    // identities decide.
     const uint32_t tkey = cand ? (t == 0.0f ? 0u : __float_as_uint(t)) : 0xffffffffu;
-    // Shared-memory minima per owner, one key at a time (the slots start
-    // at ~0 and are reset by their owners after the round). Grouping the
-    // lanes by owner with a warp match instead measured 30 % slower.
     if (cand) atomicMin(&sm.key[owner], tkey);
     __syncwarp();
     const bool c2 = cand && sm.key[owner] == tkey;
-    if (c2) atomicMin(&sm.key2[owner], inst);
+    if (c2) atomicMin(&sm.winner[owner], lane);
     __syncwarp();
-    const bool c3 = c2 && sm.key2[owner] == inst;
-    if (c3) atomicMin(&sm.winner[owner], prim);
-    __syncwarp();
-    const bool win = c3 && sm.winner[owner] == prim;
-    __syncwarp();
-    if (win) sm.winner[owner] = lane;
-    const uint32_t hasw = __ballot_sync(TQ_FULL, sm.key[lane] != 0xffffffffu);
-    __syncwarp();
-    // Each owner takes its winner's candidate over shuffles.
-    const bool mine = (hasw >> lane) & 1u;
-    const uint32_t from = mine ? sm.winner[lane] : lane;
-    const float wt = __shfl_sync(TQ_FULL, t, from), wb1 = __shfl_sync(TQ_FULL, b1, from),
-                wb2 = __shfl_sync(TQ_FULL, b2, from);
-    const uint32_t wi = __shfl_sync(TQ_FULL, inst, from), wp = __shfl_sync(TQ_FULL, prim, from);
-    if (mine && (wt < c.tmax || (wt == c.tmax && (wi < c.inst || (wi == c.inst && wp < c.prim))))) {
-        c.tmax = wt;
-        c.inst = wi;
-        c.prim = wp;
-        c.b1 = wb1;
-        c.b2 = wb2;
+    bool win = c2 && sm.winner[owner] == lane;
+    if (__any_sync(TQ_FULL, c2 && !win)) {
+        if (c2) sm.winner[owner] = sm.key2[owner] = 0xffffffffu;
+        __syncwarp();
+        if (c2) atomicMin(&sm.key2[owner], inst);
+        __syncwarp();
+        const bool c3 = c2 && sm.key2[owner] == inst;
+        if (c3) atomicMin(&sm.winner[owner], prim);
+        __syncwarp();
+        win = c3 && sm.winner[owner] == prim;
+        __syncwarp();
+        if (win) sm.winner[owner] = lane;
     }
-    sm.key[lane] = 0xffffffffu;
-    sm.key2[lane] = 0xffffffffu;
-    sm.winner[lane] = 0xffffffffu;
+    // The winner commits to its owner's slot unless the hit there has the
+    // same t and the smaller identity; the owner takes the new bound.
+    if (win) {
+        bool better = t < tmo;
+        if (!better) {
+            const uint4 cur = sm.best[owner];
+            better = inst < cur.x || (inst == cur.x && prim < cur.y);
+        }
+        if (better) sm.best[owner] = make_uint4(inst, prim, __float_as_uint(b1), __float_as_uint(b2));
+    }
+    __syncwarp();
+    const uint32_t from = sm.winner[lane];
+    const bool mine = from != 0xffffffffu;
+    const float wt = __shfl_sync(TQ_FULL, t, mine ? from : lane);
+    if (mine) {
+        if (wt < tmax) tmax = wt;
+        sm.key[lane] = 0xffffffffu;
+        sm.winner[lane] = 0xffffffffu;
+    }
     __syncwarp();
 }
 
@@ -225,38 +248,49 @@ __device__ __forceinline__ void tq_round(const DeviceScene& s, TriQueueSmem& sm,
 //   uint32_t next(bool live, bool& drained)  an item for each idle lane (~0u: none)
 //   void ray(uint32_t item, float3& org, float3& dir)      (per lane)
 //   void emit(uint32_t item, uint4 hit, float t)          (per lane)
-//   void step(bool finished, uint32_t item, uint32_t instance, float t)  after every step
+//   void step(bool finished, uint32_t item, uint32_t instance, float t)  before every refill
 //   uint32_t want_idle(bool drained)  idle lanes before the warp refills
 // Each step a walking lane expands one node and queues the triangles of the
 // leaves it hits; rounds run while the FIFO holds a warp's worth of
 // triangles, while TQ_WAITING lanes wait on it, or until it is empty once no
-// lane has nodes left. A lane whose
-// walk has ended completes when its last queued entry has been tested.
+// lane has nodes left. A lane whose walk has ended completes when its last
+// queued entry has been tested; the finished lanes are retired together
+// before the warp refills, so the stores and the sort's key counts run once
+// per refill and not at every step that ends a ray.
 // Sets `overflow` when a walk hit its iteration or stack bound.
 template <bool COUNT, class Src, int S = TRAVERSAL_STACK>
 __device__ __forceinline__ void queued_closest(const DeviceScene& s, TriQueueSmem& sm, Src& src, uint32_t ray_mask,
                                                bool& overflow, uint32_t* visits, uint32_t* tests) {
+    const uint32_t lane = threadIdx.x & 31u;
     TriQueue q{0u, 0u, 0u};
     uint2 stack[S];
     Walk w;
-    Ray ray;
-    Closest c;
-    closest_begin(c);
+    WalkRay ray{f3(0.0f), f3(0.0f), 0u};
+    float tmax = 1e30f;
     uint32_t item = 0u, last_seq = 0u;
-    bool live = false, walking = false, drained = false;
-    sm.key[threadIdx.x & 31u] = 0xffffffffu;
-    sm.key2[threadIdx.x & 31u] = 0xffffffffu;
-    sm.winner[threadIdx.x & 31u] = 0xffffffffu;
+    bool live = false, walking = false, drained = false, finished = false;
+    sm.key[lane] = 0xffffffffu;
+    sm.winner[lane] = 0xffffffffu;
     __syncwarp();
     for (;;) {
+        uint32_t inst = 0u;
+        if (finished) {
+            const uint4 hit = sm.best[lane];
+            inst = hit.x;
+            src.emit(item, hit, tmax);
+        }
+        src.step(finished, item, inst, tmax);
+        finished = false;
         if (!drained) {
             const uint32_t i = src.next(live, drained);
             if (i != ~0u) {
                 float3 o, d;
                 src.ray(i, o, d);
-                ray = make_ray(o, d);
-                closest_begin(c);
-                walk_begin(w, ray);
+                const Ray r = make_ray(o, d);
+                ray = tq_ray(sm, r);
+                sm.best[lane] = make_uint4(LIGHT_NONE, 0u, 0u, 0u);
+                tmax = 1e30f;
+                walk_begin(w, r);
                 item = i;
                 last_seq = 0u;
                 live = true;
@@ -271,7 +305,7 @@ __device__ __forceinline__ void queued_closest(const DeviceScene& s, TriQueueSme
         for (;;) {
             uint2 grp = make_uint2(0u, 0u);
             if (live && walking) {
-                if (++w.iter > walk_bound(s) || !expand_node<COUNT, S>(s, ray, c.tmax, w, stack, visits)) {
+                if (++w.iter > walk_bound(s) || !expand_node<COUNT, S>(s, ray, tmax, w, stack, visits)) {
                     overflow = true;
                     walking = false;
                 } else {
@@ -286,14 +320,11 @@ __device__ __forceinline__ void queued_closest(const DeviceScene& s, TriQueueSme
             const bool any_walking = __any_sync(TQ_FULL, live && walking);
             const bool many_waiting = uint32_t(__popc(__ballot_sync(TQ_FULL, live && !walking))) >= TQ_WAITING;
             while (q.tris >= 32u || (q.tris > 0u && (!any_walking || many_waiting)))
-                tq_round<COUNT>(s, sm, q, ray, c, ray_mask, tests);
-            bool finished = false;
+                tq_round<COUNT>(s, sm, q, ray, tmax, ray_mask, tests);
             if (live && !walking && q.head >= last_seq) {
-                src.emit(item, make_uint4(c.inst, c.prim, __float_as_uint(c.b1), __float_as_uint(c.b2)), c.tmax);
                 finished = true;
                 live = false;
             }
-            src.step(finished, item, c.inst, c.tmax);
             if (uint32_t(__popc(__ballot_sync(TQ_FULL, !live))) >= want_idle) break;
         }
     }
@@ -301,13 +332,13 @@ __device__ __forceinline__ void queued_closest(const DeviceScene& s, TriQueueSme
 
 // ---- shadow queries (trace_shadow.slang:29-72) ------------------------------------
 
-// A shadow query as the queued walk keeps it: its bound (the target
-// triangle's distance, or tmax without one), the target's leaf (~0 when the
-// target was not hit or there is none) and (instance, primitive) identity.
+// A shadow query as its source sets it up: its bound (the target triangle's
+// distance, or tmax without one), the target's leaf (~0 when the target was
+// not hit or there is none) and (instance, primitive) identity. The walk
+// keeps the bound in a register and the target in shared memory.
 struct AnyQuery {
     float tm;
     uint32_t leaf, light, lprim;
-    bool occluded;
 };
 
 // One any-hit round: each lane's triangle tested against its owner's query;
@@ -315,28 +346,30 @@ struct AnyQuery {
 // (instance, primitive) key) occludes it, as in shadow_step. All 32 lanes
 // call it together with q.tris > 0.
 template <bool COUNT = false>
-__device__ __forceinline__ void tq_round_any(const DeviceScene& s, TriQueueSmem& sm, TriQueue& q, const Ray& ray,
-                                             AnyQuery& a, uint32_t* tests) {
+__device__ __forceinline__ void tq_round_any(const DeviceScene& s, TriQueueSmem& sm, TriQueue& q, const WalkRay& ray,
+                                             float tm, bool& occluded, uint32_t* tests) {
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t dead = __ballot_sync(TQ_FULL, a.occluded);
+    const uint32_t dead = __ballot_sync(TQ_FULL, occluded);
     const TqWork wk = tq_take(sm, q);
     const uint32_t owner = wk.owner;
-    const Ray ro = owner_ray(ray, owner);
-    const float tmo = __shfl_sync(TQ_FULL, a.tm, owner);
-    const uint32_t leaf = __shfl_sync(TQ_FULL, a.leaf, owner), light = __shfl_sync(TQ_FULL, a.light, owner),
-                   lprim = __shfl_sync(TQ_FULL, a.lprim, owner);
+    const Ray ro = owner_ray(sm, ray, owner);
+    const float tmo = __shfl_sync(TQ_FULL, tm, owner);
     bool occl = false;
-    if (wk.act && !((dead >> owner) & 1u) && wk.tri != leaf && wk.tri < s.tri_count) {
-        const float4* tp = s.tris + 3u * wk.tri;
-        const float4 v0 = __ldg(tp), v1 = __ldg(tp + 1), v2 = __ldg(tp + 2);
-        if (COUNT) ++*tests;
-        float t, b1, b2;
-        if (tri_hit(ro, v0, v1, v2, tmo, t, b1, b2)) {
-            const uint32_t inst = __float_as_uint(v0.w), prim = __float_as_uint(v1.w);
-            occl = !(leaf != 0xffffffffu && t == tmo && !(inst < light || (inst == light && prim < lprim)));
+    if (wk.act && !((dead >> owner) & 1u) && wk.tri < s.tri_count) {
+        const uint4 target = sm.best[owner];  // leaf, instance, primitive
+        if (wk.tri != target.x) {
+            const float4* tp = s.tris + 3u * wk.tri;
+            const float4 v0 = __ldg(tp), v1 = __ldg(tp + 1), v2 = __ldg(tp + 2);
+            if (COUNT) ++*tests;
+            float t, b1, b2;
+            if (tri_hit(ro, v0, v1, v2, tmo, t, b1, b2)) {
+                const uint32_t inst = __float_as_uint(v0.w), prim = __float_as_uint(v1.w);
+                occl = !(target.x != 0xffffffffu && t == tmo &&
+                         !(inst < target.y || (inst == target.y && prim < target.z)));
+            }
         }
     }
-    if ((__reduce_or_sync(TQ_FULL, occl ? (1u << owner) : 0u) >> lane) & 1u) a.occluded = true;
+    if ((__reduce_or_sync(TQ_FULL, occl ? (1u << owner) : 0u) >> lane) & 1u) occluded = true;
     __syncwarp();
 }
 
@@ -346,38 +379,49 @@ __device__ __forceinline__ void tq_round_any(const DeviceScene& s, TriQueueSmem&
 //   uint32_t next(bool live, bool& drained)  an item for each idle lane (~0u: none)
 //   bool begin(uint32_t item, Ray& ray, AnyQuery& a)   (per lane) false: the
 //       query has no target leaf to bound it; then `closest(item)` answers it
-//       with the per-lane closest-hit walk
+//       with the per-lane closest-hit walk (only where FALLBACK is set)
 //   template <int S> void closest(uint32_t item, uint2* stack)  (per lane; the
 //       stack holds S entries)
 //   void emit(uint32_t item, bool visible)              (per lane; a query
 //       whose walk hit a bound counts as occluded)
 //   uint32_t want_idle(bool drained)
 // An occluded query stops walking at once; its entries still queued are
-// skipped, and it completes when they have left the queue.
+// skipped, and it completes when they have left the queue. Finished queries
+// are retired together before the warp refills.
 template <bool COUNT, class Src, int S = TRAVERSAL_STACK>
 __device__ __forceinline__ void queued_any(const DeviceScene& s, TriQueueSmem& sm, Src& src, bool& overflow,
                                            uint32_t* visits, uint32_t* tests) {
+    const uint32_t lane = threadIdx.x & 31u;
     TriQueue q{0u, 0u, 0u};
     uint2 stack[S];
     Walk w;
-    Ray ray;
-    AnyQuery a{0.0f, 0xffffffffu, LIGHT_NONE, 0u, false};
+    WalkRay ray{f3(0.0f), f3(0.0f), 0u};
+    float tm = 0.0f;
     uint32_t item = 0u, last_seq = 0u;
-    bool live = false, walking = false, drained = false, ovf = false;
+    bool live = false, walking = false, drained = false, occluded = false, finished = false;
     for (;;) {
+        if (finished) src.emit(item, !occluded);
+        finished = false;
         if (!drained) {
             const uint32_t i = src.next(live, drained);
             if (i != ~0u) {
                 item = i;
                 last_seq = 0u;
                 live = true;
-                ovf = false;
-                walking = src.begin(i, ray, a) && s.node_count != 0;
-                if (!walking && !a.occluded && s.node_count != 0) {
-                    src.template closest<S>(i, stack);  // no target leaf: the per-lane closest-hit query
-                    live = false;
+                occluded = false;
+                Ray r;
+                AnyQuery a;
+                walking = src.begin(i, r, a) && s.node_count != 0;
+                if constexpr (Src::FALLBACK) {
+                    if (!walking && s.node_count != 0) {
+                        src.template closest<S>(i, stack);  // no target leaf: the per-lane closest-hit query
+                        live = false;
+                    }
                 }
-                walk_begin(w, ray);
+                ray = tq_ray(sm, r);
+                tm = a.tm;
+                sm.best[lane] = make_uint4(a.leaf, a.light, a.lprim, 0u);
+                walk_begin(w, r);
             }
         }
         if (!__any_sync(TQ_FULL, live)) {
@@ -387,10 +431,10 @@ __device__ __forceinline__ void queued_any(const DeviceScene& s, TriQueueSmem& s
         const uint32_t want_idle = src.want_idle(drained);
         for (;;) {
             uint2 grp = make_uint2(0u, 0u);
-            if (live && walking && !a.occluded) {
-                if (++w.iter > walk_bound(s) || !expand_node<COUNT, S>(s, ray, a.tm, w, stack, visits)) {
+            if (live && walking && !occluded) {
+                if (++w.iter > walk_bound(s) || !expand_node<COUNT, S>(s, ray, tm, w, stack, visits)) {
                     overflow = true;
-                    ovf = true;  // dropped, as the per-lane walk drops it
+                    occluded = true;  // dropped, as the per-lane walk drops it
                     walking = false;
                 } else {
                     grp = w.t;
@@ -401,10 +445,11 @@ __device__ __forceinline__ void queued_any(const DeviceScene& s, TriQueueSmem& s
                 }
             }
             tq_append(sm, q, grp, last_seq);
-            const bool any_walking = __any_sync(TQ_FULL, live && walking && !a.occluded);
-            while (q.tris >= 32u || (q.tris > 0u && !any_walking)) tq_round_any<COUNT>(s, sm, q, ray, a, tests);
-            if (live && (!walking || a.occluded) && q.head >= last_seq) {
-                src.emit(item, !a.occluded && !ovf);
+            const bool any_walking = __any_sync(TQ_FULL, live && walking && !occluded);
+            while (q.tris >= 32u || (q.tris > 0u && !any_walking))
+                tq_round_any<COUNT>(s, sm, q, ray, tm, occluded, tests);
+            if (live && (!walking || occluded) && q.head >= last_seq) {
+                finished = true;
                 live = false;
             }
             if (uint32_t(__popc(__ballot_sync(TQ_FULL, !live))) >= want_idle) break;

@@ -263,11 +263,17 @@ __global__ void __launch_bounds__(B, CN_ISECT_MIN_BLOCKS * BLOCK / B)
     uint32_t path = 0, best_inst = LIGHT_NONE, best_prim = 0, crossings = 0, pixel = 0, sample = 0;
     uint32_t qi = 0;          // the ray's queue position (the material sort's key slot)
     bool live = false, drained = false, finished = false;
-    // Material sort (when this bounce sorts): each finished ray's key goes to
-    // its queue slot and into the key counts, one atomic per distinct key per
-    // warp. Called where the whole warp is converged.
-    auto flush_keys = [&]() {
-        if (!pool.sort_keys) return;
+    // The rays that finished since the last refill: their hits and, when this
+    // bounce sorts, their keys (to their queue slots and into the key counts,
+    // one atomic per distinct key per warp). Called where the whole warp is
+    // converged.
+    auto retire = [&]() {
+        if (finished)
+            pool.hit[path] = make_uint4(best_inst, best_prim, __float_as_uint(best_b1), __float_as_uint(best_b2));
+        if (!pool.sort_keys) {
+            finished = false;
+            return;
+        }
         if (__ballot_sync(0xffffffffu, finished) == 0u) return;
         const uint32_t key = finished ? material_key(scene, pool, best_inst, path, tmax) : 0xffffffffu;
         const uint32_t peers = __match_any_sync(0xffffffffu, key);
@@ -298,6 +304,7 @@ __global__ void __launch_bounds__(B, CN_ISECT_MIN_BLOCKS * BLOCK / B)
         return false;
     };
     for (;;) {
+        retire();
         if (!drained) {
             uint32_t i = refill(fetch, count, live, drained);
             if (i != ~0u) {
@@ -318,16 +325,15 @@ __global__ void __launch_bounds__(B, CN_ISECT_MIN_BLOCKS * BLOCK / B)
                 walk_begin(w, ray);
                 live = true;
                 if (scene.node_count == 0) {
-                    pool.hit[path] = make_uint4(LIGHT_NONE, 0u, 0u, 0u);
                     live = false;
                     finished = true;
                 }
             }
         }
-        flush_keys();
         if (!__any_sync(0xffffffffu, live)) {
-            if (drained) break;
-            continue;
+            if (!drained) continue;
+            retire();
+            break;
         }
         // Walk until enough lanes are idle to refill (all of them once drained).
         const uint32_t want_idle = drained ? 32u : (pool.refill_idle ? pool.refill_idle : uint32_t(CN_REFILL_IDLE));
@@ -336,13 +342,10 @@ __global__ void __launch_bounds__(B, CN_ISECT_MIN_BLOCKS * BLOCK / B)
                 int st = walk_step<COUNT, S>(scene, ray, tmax, w, stack, visit, &visits, &tests);
                 if (st != WALK_CONTINUE) {
                     if (st == WALK_OVERFLOW) flag_overflow(pool.counters);
-                    pool.hit[path] =
-                        make_uint4(best_inst, best_prim, __float_as_uint(best_b1), __float_as_uint(best_b2));
                     live = false;
                     finished = true;
                 }
             }
-            flush_keys();
             if (uint32_t(__popc(__ballot_sync(0xffffffffu, !live))) >= want_idle) break;
         }
     }
@@ -843,6 +846,9 @@ __global__ void __launch_bounds__(B, CN_TRAV_MIN_BLOCKS * BLOCK / B)
 // persistent, refilling grid with the triangle tests shared by the warp
 // through its triangle queue (trqueue.cuh). Radiance is bitwise k_shadow's.
 struct ShadowSource {
+    // Every connection's target has a leaf: scene creation looks up the leaf of
+    // each emissive triangle, and all triangles are in the tree.
+    static constexpr bool FALLBACK = false;
     const DeviceScene& scene;
     const PathPool& pool;
     uint32_t* fetch;
@@ -853,12 +859,10 @@ struct ShadowSource {
         const float4 q0 = rec[0], q1 = rec[1], q2 = rec[2], q3 = rec[3];
         ray = make_ray(xyz(q0), xyz(q1));
         const uint32_t light = __float_as_uint(q2.w), leaf = __float_as_uint(q3.y);
-        a.occluded = false;
         a.light = light;
         a.lprim = __float_as_uint(q3.x);
         a.tm = q0.w;
         a.leaf = 0xffffffffu;
-        if (light != LIGHT_NONE && leaf == 0xffffffffu) return false;  // no leaf: the closest-hit query
         if (leaf < scene.tri_count) {
             const float4* tp = scene.tris + 3u * leaf;
             float t, b1, b2;
@@ -874,15 +878,6 @@ struct ShadowSource {
         const uint32_t path = __float_as_uint(rec[1].w);
         const float4 c = rec[2], r = pool.rad[path];
         pool.rad[path] = make_float4(r.x + c.x * atten, r.y + c.y * atten, r.z + c.z * atten, r.w);
-    }
-    template <int S>
-    __device__ __forceinline__ void closest(uint32_t i, uint2* stack) const {
-        const float4* rec = reinterpret_cast<const float4*>(pool.shadows + i);
-        const float4 q0 = rec[0], q1 = rec[1], q2 = rec[2], q3 = rec[3];
-        const float atten = shadow_query<false, S>(scene, make_ray(xyz(q0), xyz(q1)), q0.w, __float_as_uint(q2.w),
-                                                   __float_as_uint(q3.x), __float_as_uint(q3.y), stack);
-        if (atten == -2.0f) flag_overflow(pool.counters);
-        else if (atten >= 0.0f) add(i, atten);
     }
     __device__ __forceinline__ void emit(uint32_t i, bool visible) const {
         if (visible) add(i, 1.0f);
