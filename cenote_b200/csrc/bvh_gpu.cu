@@ -933,6 +933,37 @@ __global__ void k_light_leaves(const float4* __restrict__ tris, uint32_t n, cons
     }
 }
 
+// One thread per triangle of the concatenated meshes: its instance by binary
+// search, its corners gathered through the instance's indices.
+__global__ void k_attributes(const float* __restrict__ positions, const float* __restrict__ normals,
+                             const float* __restrict__ uvs, const uint32_t* __restrict__ indices,
+                             const uint32_t* __restrict__ first_tri, const uint64_t* __restrict__ first_vertex,
+                             uint32_t instances, uint32_t n, float4* __restrict__ attrs) {
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+        uint32_t lo = 0, hi = instances;  // the last instance starting at or before t
+        while (hi - lo > 1) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (__ldg(first_tri + mid) <= t) lo = mid;
+            else hi = mid;
+        }
+        const size_t base = first_vertex[lo];
+        float uv[6];
+        float4* out = attrs + size_t(t) * TRI_ATTRS;
+        size_t v[3];
+        for (int k = 0; k < 3; ++k) {
+            v[k] = base + __ldg(indices + 3 * size_t(t) + k);
+            uv[2 * k] = __ldg(uvs + 2 * v[k]);
+            uv[2 * k + 1] = __ldg(uvs + 2 * v[k] + 1);
+        }
+        for (int k = 0; k < 3; ++k) {
+            const float* p = positions + 3 * v[k];
+            const float* q = normals + 3 * v[k];
+            out[k] = make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), uv[k]);
+            out[3 + k] = make_float4(__ldg(q), __ldg(q + 1), __ldg(q + 2), uv[3 + k]);
+        }
+    }
+}
+
 int grid_for(uint32_t n) {
     uint32_t g = (n + BLOCK - 1) / BLOCK;
     return int(g < 1 ? 1 : (g > 148u * 32u ? 148u * 32u : g));
@@ -1260,6 +1291,14 @@ cudaError_t build_wide_bvh_gpu(const float4* in, uint32_t n, GpuBvh* out, cudaSt
 void launch_light_leaves(const float4* tris, uint32_t n, const GeomRecord* geometry, uint32_t* light_leaf,
                          cudaStream_t s) {
     if (n) k_light_leaves<<<grid_for(n), BLOCK, 0, s>>>(tris, n, geometry, light_leaf);
+}
+
+void launch_attributes(const float* positions, const float* normals, const float* uvs, const uint32_t* indices,
+                       const uint32_t* first_tri, const uint64_t* first_vertex, uint32_t instances, uint32_t n,
+                       float4* attrs, cudaStream_t s) {
+    if (n)
+        k_attributes<<<grid_for(n), BLOCK, 0, s>>>(positions, normals, uvs, indices, first_tri, first_vertex, instances,
+                                                   n, attrs);
 }
 
 }  // namespace cn

@@ -25,4 +25,11 @@ cudaError_t build_wide_bvh_gpu(const float4* in, uint32_t n, GpuBvh* out, cudaSt
 void launch_light_leaves(const float4* tris, uint32_t n, const GeomRecord* geometry, uint32_t* light_leaf,
                          cudaStream_t s);
 
+// Every triangle's attribute record (TRI_ATTRS float4 each) from `n` triangles
+// of concatenated meshes: instance i's indices start at triangle first_tri[i]
+// (first_tri[instances] = n) and count from its vertex first_vertex[i].
+void launch_attributes(const float* positions, const float* normals, const float* uvs, const uint32_t* indices,
+                       const uint32_t* first_tri, const uint64_t* first_vertex, uint32_t instances, uint32_t n,
+                       float4* attrs, cudaStream_t s);
+
 }  // namespace cn

@@ -446,6 +446,19 @@ int32_t cenote_scene_create_textured(cenote_context* ctx, const cenote_object* o
     size_t total_tris = 0;
     for (uint32_t i = 0; i < object_count; ++i) total_tris += objects[i].triangle_count;
     tris.reserve(total_tris);
+    // Every mesh's vertices and indices end to end: one upload per stream, from
+    // which the device writes the triangles' attribute records.
+    std::vector<uint32_t> first_tri(size_t(object_count) + 1, 0);
+    std::vector<uint64_t> first_vertex(object_count, 0);
+    size_t total_vertices = 0;
+    for (uint32_t i = 0; i < object_count; ++i) total_vertices += objects[i].vertex_count;
+    CN_CHECK(total_tris < (1ull << 32), CENOTE_E_SCENE, "the scene's triangles exceed 32 bits");
+    std::vector<float> positions, normals, uvs;
+    std::vector<uint32_t> indices;
+    positions.reserve(3 * total_vertices);
+    normals.reserve(3 * total_vertices);
+    uvs.reserve(2 * total_vertices);
+    indices.reserve(3 * total_tris);
     bool nonopaque = false, layered = false;
     for (uint32_t i = 0; i < object_count; ++i) {
         const cenote_object& o = objects[i];
@@ -460,24 +473,12 @@ int32_t cenote_scene_create_textured(cenote_context* ctx, const cenote_object* o
         CN_CHECK(invert_affine(o.transform, g.w2o), CENOTE_E_INVALID_ARGUMENT,
                  "object " + std::to_string(i) + " transform is not invertible");
         g.light = LIGHT_NONE;
-        DeviceBuffer* bp = sc->add(size_t(o.vertex_count) * 12, &err);
-        CN_CUDA(err);
-        DeviceBuffer* bn = sc->add(size_t(o.vertex_count) * 12, &err);
-        CN_CUDA(err);
-        DeviceBuffer* bu = sc->add(size_t(o.vertex_count) * 8, &err);
-        CN_CUDA(err);
-        DeviceBuffer* bi = sc->add(size_t(o.triangle_count) * 12, &err);
-        CN_CUDA(err);
-        CN_CUDA(cudaMemcpyAsync(bp->ptr, o.positions, size_t(o.vertex_count) * 12, cudaMemcpyHostToDevice, ctx->stream));
-        CN_CUDA(cudaMemcpyAsync(bn->ptr, o.normals, size_t(o.vertex_count) * 12, cudaMemcpyHostToDevice, ctx->stream));
-        CN_CUDA(cudaMemcpyAsync(bu->ptr, o.uvs, size_t(o.vertex_count) * 8, cudaMemcpyHostToDevice, ctx->stream));
-        if (o.triangle_count)
-            CN_CUDA(cudaMemcpyAsync(bi->ptr, o.indices, size_t(o.triangle_count) * 12, cudaMemcpyHostToDevice,
-                                    ctx->stream));
-        g.positions = bp->as<float>();
-        g.normals = bn->as<float>();
-        g.uvs = bu->as<float>();
-        g.indices = bi->as<uint32_t>();
+        first_vertex[i] = positions.size() / 3;
+        first_tri[i + 1] = first_tri[i] + o.triangle_count;
+        positions.insert(positions.end(), o.positions, o.positions + 3 * size_t(o.vertex_count));
+        normals.insert(normals.end(), o.normals, o.normals + 3 * size_t(o.vertex_count));
+        uvs.insert(uvs.end(), o.uvs, o.uvs + 2 * size_t(o.vertex_count));
+        indices.insert(indices.end(), o.indices, o.indices + 3 * size_t(o.triangle_count));
         mats[i] = o.material;
         V3 em = v3(o.material.emission);
         bool emissive = em.x != 0.0f || em.y != 0.0f || em.z != 0.0f;
@@ -522,6 +523,26 @@ int32_t cenote_scene_create_textured(cenote_context* ctx, const cenote_object* o
     DeviceBuffer* btris = nullptr;
     uint32_t node_count = 0;
     const uint32_t tri_count = uint32_t(tris.size());
+    DeviceBuffer* battrs = sc->add(size_t(tri_count) * TRI_ATTRS * 16, &err);
+    CN_CUDA(err);
+    DeviceBuffer mesh_stage[6];
+    {
+        const std::pair<const void*, size_t> streams[6] = {
+            {positions.data(), positions.size() * 4}, {normals.data(), normals.size() * 4},
+            {uvs.data(), uvs.size() * 4},             {indices.data(), indices.size() * 4},
+            {first_tri.data(), first_tri.size() * 4}, {first_vertex.data(), first_vertex.size() * 8}};
+        for (int k = 0; k < 6; ++k) {
+            CN_CUDA(mesh_stage[k].alloc(streams[k].second));
+            if (streams[k].second)
+                CN_CUDA(cudaMemcpyAsync(mesh_stage[k].ptr, streams[k].first, streams[k].second, cudaMemcpyHostToDevice,
+                                        ctx->stream));
+        }
+        launch_attributes(mesh_stage[0].as<float>(), mesh_stage[1].as<float>(), mesh_stage[2].as<float>(),
+                          mesh_stage[3].as<uint32_t>(), mesh_stage[4].as<uint32_t>(), mesh_stage[5].as<uint64_t>(),
+                          object_count, tri_count, battrs->as<float4>(), ctx->stream);
+        CN_CUDA(cudaGetLastError());
+    }
+    for (uint32_t i = 0; i < object_count; ++i) geoms[i].attrs = battrs->as<float4>() + size_t(first_tri[i]) * TRI_ATTRS;
     DeviceBuffer* bgeo = sc->add(geoms.size() * sizeof(GeomRecord), &err);
     CN_CUDA(err);
     CN_CUDA(cudaMemcpyAsync(bgeo->ptr, geoms.data(), geoms.size() * sizeof(GeomRecord), cudaMemcpyHostToDevice,

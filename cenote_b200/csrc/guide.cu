@@ -462,18 +462,14 @@ __global__ void k_cast(const float* __restrict__ p, __nv_bfloat16* __restrict__ 
 
 // ---- in the wavefront ------------------------------------------------------------------------
 
-__device__ __forceinline__ float3 ld3(const float* p, uint32_t v) {
-    return make_float3(__ldg(p + 3 * v), __ldg(p + 3 * v + 1), __ldg(p + 3 * v + 2));
-}
-
 // A hit's world position and geometric normal turned against the ray: the
 // guide's inputs (the shading kernel records the same quantities).
 __device__ void hit_frame(const DeviceScene& s, uint4 h, float3 dir, float3& pos, float3& nrm) {
     const GeomRecord& g = s.geometry[h.x];
     const uint32_t prim = h.y;
     const float b1 = __uint_as_float(h.z), b2 = __uint_as_float(h.w);
-    uint32_t i0 = __ldg(g.indices + 3 * prim), i1 = __ldg(g.indices + 3 * prim + 1), i2 = __ldg(g.indices + 3 * prim + 2);
-    float3 v0 = ld3(g.positions, i0), v1 = ld3(g.positions, i1), v2 = ld3(g.positions, i2);
+    const float4* at = g.attrs + size_t(prim) * TRI_ATTRS;
+    const float4 v0 = __ldg(at), v1 = __ldg(at + 1), v2 = __ldg(at + 2);
     float3 e1 = make_float3(v1.x - v0.x, v1.y - v0.y, v1.z - v0.z), e2 = make_float3(v2.x - v0.x, v2.y - v0.y, v2.z - v0.z);
     float3 op = make_float3(v0.x + b1 * e1.x + b2 * e2.x, v0.y + b1 * e1.y + b2 * e2.y, v0.z + b1 * e1.z + b2 * e2.z);
     float3 on = make_float3(e1.y * e2.z - e1.z * e2.y, e1.z * e2.x - e1.x * e2.z, e1.x * e2.y - e1.y * e2.x);

@@ -47,18 +47,26 @@ struct LightRecord {
 };
 static_assert(sizeof(LightRecord) == 80, "light record is 80 bytes");
 
-// Everything shading needs to re-evaluate a hit on one instance: its
-// object-space attributes, both transforms, and its first light record.
-struct GeomRecord {
-    const float* positions;
-    const float* normals;
-    const float* uvs;
-    const uint32_t* indices;
+// Everything shading needs to re-evaluate a hit on one instance: both
+// transforms, its triangles' object-space attributes and its first light
+// record.
+//
+// The attributes are stored per triangle, TRI_ATTRS float4 each (96 bytes,
+// three whole sectors): position k in lane xyz of float4 k, normal k in lane
+// xyz of float4 3 + k, and the UVs' six floats in the w lanes in order. A hit
+// reads them with six 16-byte loads at an address known from (instance,
+// primitive). Through an index buffer and three vertex arrays the same values
+// took 27 scalar loads, the vertices' waiting on the indices', from up to a
+// dozen lines: shading was bound by those gathers.
+constexpr uint32_t TRI_ATTRS = 6;
+struct alignas(16) GeomRecord {
     float o2w[3][4];
     float w2o[3][4];
+    const float4* attrs;
     uint32_t light;
-    uint32_t pad[3];
+    uint32_t pad;
 };
+static_assert(sizeof(GeomRecord) == 112, "geometry record is 112 bytes");
 
 // Compressed wide BVH node (Ylitie, Karras & Laine, HPG 2017): 80 bytes =
 // five 16-byte vector loads. Child boxes are 8-bit offsets from `p` in units

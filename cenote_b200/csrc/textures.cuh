@@ -32,23 +32,48 @@ __device__ __forceinline__ float3 sample_normal(const DeviceScene& s, uint32_t i
     return f3(x, y, sqrtf(fmaxf(1.0f - (x * x + y * y), 0.0f)));
 }
 
-// scene.slang:31-37, from the instance's own index and UV streams.
-__device__ __forceinline__ float2 interpolate_uv(const float* uvs, const uint32_t* indices, uint32_t prim, float b1,
-                                                 float b2) {
-    uint32_t i0 = __ldg(indices + 3 * prim), i1 = __ldg(indices + 3 * prim + 1), i2 = __ldg(indices + 3 * prim + 2);
-    float2 u0 = __ldg(reinterpret_cast<const float2*>(uvs) + i0);
-    float2 u1 = __ldg(reinterpret_cast<const float2*>(uvs) + i1);
-    float2 u2 = __ldg(reinterpret_cast<const float2*>(uvs) + i2);
+// One triangle's attribute record (GeomRecord::attrs).
+struct TriAttrs {
+    float4 a[TRI_ATTRS];
+    __device__ __forceinline__ float3 position(int k) const { return xyz(a[k]); }
+    __device__ __forceinline__ float3 normal(int k) const { return xyz(a[3 + k]); }
+    __device__ __forceinline__ float2 uv(int k) const { return make_float2(a[2 * k].w, a[2 * k + 1].w); }
+};
+
+__device__ __forceinline__ TriAttrs load_attrs(const float4* attrs, uint32_t prim) {
+    TriAttrs t;
+    const float4* p = attrs + size_t(prim) * TRI_ATTRS;
+#pragma unroll
+    for (uint32_t k = 0; k < TRI_ATTRS; ++k) t.a[k] = __ldg(p + k);
+    return t;
+}
+
+// The UVs alone.
+struct TriUvs {
+    float f[2 * 3];
+    __device__ __forceinline__ float2 uv(int k) const { return make_float2(f[2 * k], f[2 * k + 1]); }
+};
+
+__device__ __forceinline__ TriUvs load_uvs(const float4* attrs, uint32_t prim) {
+    TriUvs t;
+    const float* p = reinterpret_cast<const float*>(attrs + size_t(prim) * TRI_ATTRS);
+#pragma unroll
+    for (uint32_t k = 0; k < TRI_ATTRS; ++k) t.f[k] = __ldg(p + 4 * k + 3);
+    return t;
+}
+
+// scene.slang:31-37.
+template <class T>
+__device__ __forceinline__ float2 interpolate_uv(const T& t, float b1, float b2) {
+    const float2 u0 = t.uv(0), u1 = t.uv(1), u2 = t.uv(2);
     return make_float2(u0.x + b1 * (u1.x - u0.x) + b2 * (u2.x - u0.x), u0.y + b1 * (u1.y - u0.y) + b2 * (u2.y - u0.y));
 }
 
 __device__ __forceinline__ float2 interpolate_uv(const DeviceScene& s, uint32_t inst, uint32_t prim, float b1,
                                                  float b2) {
-    const GeomRecord* g = s.geometry + inst;
-    const float* uvs = reinterpret_cast<const float*>(__ldg(reinterpret_cast<const unsigned long long*>(&g->uvs)));
-    const uint32_t* idx =
-        reinterpret_cast<const uint32_t*>(__ldg(reinterpret_cast<const unsigned long long*>(&g->indices)));
-    return interpolate_uv(uvs, idx, prim, b1, b2);
+    const float4* attrs = reinterpret_cast<const float4*>(
+        __ldg(reinterpret_cast<const unsigned long long*>(&s.geometry[inst].attrs)));
+    return interpolate_uv(load_uvs(attrs, prim), b1, b2);
 }
 
 // The slots resolveMaterial replaces (textures.slang:70-82): base colour,
@@ -122,15 +147,13 @@ static __device__ __noinline__ float3 emission_map(const DeviceScene& s, uint32_
 static __device__ __noinline__ float3 mapped_shading_normal(const DeviceScene& s, uint32_t inst, uint32_t prim,
                                                             float2 uv, uint32_t map, float3 shading, float3 normal) {
     const GeomRecord& g = s.geometry[inst];
-    uint32_t i0 = __ldg(g.indices + 3 * prim), i1 = __ldg(g.indices + 3 * prim + 1), i2 = __ldg(g.indices + 3 * prim + 2);
-    const float2* uvs = reinterpret_cast<const float2*>(g.uvs);
-    float2 u0 = __ldg(uvs + i0), u1 = __ldg(uvs + i1), u2 = __ldg(uvs + i2);
+    const TriUvs uvs = load_uvs(g.attrs, prim);
+    float2 u0 = uvs.uv(0), u1 = uvs.uv(1), u2 = uvs.uv(2);
     float du1 = u1.x - u0.x, dv1 = u1.y - u0.y, du2 = u2.x - u0.x, dv2 = u2.y - u0.y;
     float det = du1 * dv2 - dv1 * du2;
     if (fabsf(det) < 1e-12f) return shading;
-    float3 p0 = f3(__ldg(g.positions + 3 * i0), __ldg(g.positions + 3 * i0 + 1), __ldg(g.positions + 3 * i0 + 2));
-    float3 p1 = f3(__ldg(g.positions + 3 * i1), __ldg(g.positions + 3 * i1 + 1), __ldg(g.positions + 3 * i1 + 2));
-    float3 p2 = f3(__ldg(g.positions + 3 * i2), __ldg(g.positions + 3 * i2 + 1), __ldg(g.positions + 3 * i2 + 2));
+    const float4* ap = g.attrs + size_t(prim) * TRI_ATTRS;
+    float3 p0 = xyz(__ldg(ap)), p1 = xyz(__ldg(ap + 1)), p2 = xyz(__ldg(ap + 2));
     float3 e1 = p1 - p0, e2 = p2 - p0;
     float3 r0 = f3(g.o2w[0][0], g.o2w[0][1], g.o2w[0][2]), r1 = f3(g.o2w[1][0], g.o2w[1][1], g.o2w[1][2]),
            r2 = f3(g.o2w[2][0], g.o2w[2][1], g.o2w[2][2]);

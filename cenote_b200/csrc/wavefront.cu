@@ -411,14 +411,9 @@ struct Spawn {
     bool front;
 };
 
-__device__ __forceinline__ float3 fetch3(const float* a, uint32_t v) {
-    return f3(__ldg(a + 3 * v), __ldg(a + 3 * v + 1), __ldg(a + 3 * v + 2));
-}
-
 // shade_surface.slang:96-181 (van Antwerpen's rigorous spawn offsets).
-__device__ __forceinline__ Spawn spawn_point(const GeomRecord& g, uint32_t prim, float b1, float b2, float3 rd) {
-    uint32_t i0 = __ldg(g.indices + 3 * prim), i1 = __ldg(g.indices + 3 * prim + 1), i2 = __ldg(g.indices + 3 * prim + 2);
-    float3 v0 = fetch3(g.positions, i0), v1 = fetch3(g.positions, i1), v2 = fetch3(g.positions, i2);
+__device__ __forceinline__ Spawn spawn_point(const GeomRecord& g, const TriAttrs& at, float b1, float b2, float3 rd) {
+    float3 v0 = at.position(0), v1 = at.position(1), v2 = at.position(2);
     float3 e1 = v1 - v0, e2 = v2 - v0;
     float3 op = v0 + fma3(f3(b1), e1, b2 * e2);
     float3 on = cross(e1, e2);
@@ -452,7 +447,7 @@ __device__ __forceinline__ Spawn spawn_point(const GeomRecord& g, uint32_t prim,
     Spawn sp;
     sp.front = dot(wn, rd) < 0.0f;
     if (dot(wn, rd) > 0.0f) wn = -wn;
-    float3 n0 = fetch3(g.normals, i0), n1 = fetch3(g.normals, i1), n2 = fetch3(g.normals, i2);
+    float3 n0 = at.normal(0), n1 = at.normal(1), n2 = at.normal(2);
     float3 os = n0 + b1 * (n1 - n0) + b2 * (n2 - n0);
     float3 sh = normalize(w0 * os.x + w1 * os.y + w2 * os.z);
     if (dot(sh, wn) < 0.0f) sh = -sh;
@@ -554,8 +549,11 @@ __global__ void __launch_bounds__(BLOCK, LAYERS ? CN_SHADE_LAYERED_MIN_BLOCKS : 
                 float3 origin = xyz(pool.org[path]);
                 // The instance record is read field by field where used (all
                 // lanes of a sorted warp mostly share it, so the reads hit L1):
-                // a register copy of its 144 bytes made the kernel spill more.
+                // a register copy of it made the kernel spill more.
                 const GeomRecord& g = scene.geometry[inst];
+                const TriAttrs at = load_attrs(g.attrs, prim);
+                const Spawn sp0 = spawn_point(g, at, b1, b2, dir);
+                const float2 uv = interpolate_uv(at, b1, b2);
                 Material mat;
                 load_material(scene.materials + inst, mat);
                 if (!LAYERS) {
@@ -567,12 +565,8 @@ __global__ void __launch_bounds__(BLOCK, LAYERS ? CN_SHADE_LAYERED_MIN_BLOCKS : 
                 // Textured parameters resolve once at the hit's UV
                 // (shade_surface.slang:249-252).
                 const bool normal_map = mat.normal_texture != TEXTURE_NONE;
-                float2 uv = make_float2(0.0f, 0.0f);
-                if (has_parameter_maps(mat) || normal_map) {
-                    uv = interpolate_uv(g.uvs, g.indices, prim, b1, b2);
-                    resolve_material(scene, mat, uv);
-                }
-                Spawn sp = spawn_point(g, prim, b1, b2, dir);
+                if (has_parameter_maps(mat) || normal_map) resolve_material(scene, mat, uv);
+                Spawn sp = sp0;
                 if (normal_map)
                     sp.shading = mapped_shading_normal(scene, inst, prim, uv, mat.normal_texture, sp.shading, sp.normal);
                 uint32_t medium = bounce == 0 ? MEDIUM_NONE : (pool.state[path] & 0xffffffu);
