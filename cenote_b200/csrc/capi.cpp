@@ -1053,6 +1053,7 @@ int32_t run_waves(cenote_renderer* r, cenote_scene* sc, uint32_t width, uint32_t
     WavePlan plan = plan_waves(r, pixels, count, oneshot != nullptr);
     CN_CHECK(plan.need < (1ull << 31), CENOTE_E_INVALID_ARGUMENT, "wave too large");
     CN_CUDA(r->ensure(plan.need));
+    CN_CUDA(r->ensure_side(false));
     // Films trace the guides (Renderer::accumulate); one-shot renders do not.
     CN_CUDA(r->set_guides(film != nullptr));
     CN_CUDA(r->set_learned_guide(r->guide != nullptr));

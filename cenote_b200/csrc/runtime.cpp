@@ -78,13 +78,22 @@ WavePlan plan_waves(const cenote_renderer* r, uint64_t pixels, uint32_t count, b
 
 // The bounces of one wave of n0 camera paths already in the pool: per
 // bounce intersect, (the guide's inference,) the material sort, shade and
-// shadow. Timing marks bracket intersect, shade and shadow when `timing`.
+// shadow. A bounce's shadow walk runs on the renderer's side stream beside the
+// next bounce's intersect and sort, which touch nothing it reads or writes
+// (it adds to the radiance that the next shade reads): the two walks fill
+// each other's tails, and on small waves the shorter one's latency vanishes.
+// Timing marks bracket intersect, shade and shadow when `timing`, which keeps
+// them in turn on one stream.
 void enqueue_bounces(cenote_renderer* r, const cenote_scene* sc, const WaveParams& wp, uint32_t n0, bool guided,
                      cudaStream_t stream, bool timing, bool counting, WaveCounts* wc) {
     cenote_context* ctx = r->ctx;
     auto mark = [&]() {
         if (timing) cudaEventRecord(r->event(wc->events++), stream);
     };
+    int priority = 0, least = 0, greatest = 0;
+    cudaDeviceGetStreamPriorityRange(&least, &greatest);
+    cudaStreamGetPriority(stream, &priority);
+    cudaStream_t side = timing ? stream : r->side[priority < least ? 1 : 0];
     for (uint32_t b = 0; b < wp.max_bounces; ++b) {
         const bool sort = r->material_sort == CENOTE_SORT_ALL || (r->material_sort == CENOTE_SORT_SECONDARY && b > 0);
         const PathPool view = sort ? r->sorted_view() : r->pool;
@@ -100,9 +109,20 @@ void enqueue_bounces(cenote_renderer* r, const cenote_scene* sc, const WaveParam
             launch_material_sort(view, b, n0, ctx->shape, stream);
             wc->launches += sc->ds.has_layers ? 3 : 2;  // a split shading launch adds one
         }
+        if (side != stream && b > 0) cudaStreamWaitEvent(stream, r->join, 0);
         launch_shade(sc->ds, view, b, wp, n0, ctx->shape, stream);
         mark();
-        launch_shadow(sc->ds, r->pool, b, ctx->shape, counting, stream);
+        // The last bounce's shade pushes no shadow rays.
+        if (b + 1 >= wp.max_bounces) {
+            mark();
+            continue;
+        }
+        if (side != stream) {
+            cudaEventRecord(r->fork, stream);
+            cudaStreamWaitEvent(side, r->fork, 0);
+        }
+        launch_shadow(sc->ds, r->pool, b, ctx->shape, counting, side);
+        if (side != stream) cudaEventRecord(r->join, side);
         mark();
     }
 }
@@ -129,7 +149,7 @@ cudaError_t enqueue_segments(cenote_renderer* r, const cenote_scene* sc, const W
     enqueue_bounces(r, sc, wp, n0, false, stream, false, false, wc);
     launch_tally(r->pool, r->tally.as<unsigned long long>(), n0, max_bounces, stream);
     launch_accumulate_segments(r->pool, segs, nseg, items, hdr, stream);
-    wc->launches += 3 + 3 * max_bounces;
+    wc->launches += 2 + 3 * max_bounces;
     wc->waves++;
     return cudaGetLastError();
 }
@@ -210,7 +230,7 @@ cudaError_t enqueue_waves(cenote_renderer* r, const cenote_scene* sc, uint32_t w
                                                 stream);
                 }
             }
-            wc->launches += 3 + 3 * max_bounces;
+            wc->launches += 2 + 3 * max_bounces;
             wc->waves++;
         }
         done += s;

@@ -171,11 +171,30 @@ struct cenote_renderer {
     size_t g_cap = 0;
     static constexpr uint32_t GUIDE_RECORDS = 1u << 20;
     static constexpr uint32_t GUIDE_BATCH = 65536;
+    // The shadow walks' own stream (index 1: at the highest priority, beside a
+    // main stream of that priority) and the events that fork it off the main
+    // stream and join it back, every bounce of every wave.
+    cudaStream_t side[2] = {nullptr, nullptr};
+    cudaEvent_t fork = nullptr, join = nullptr;
+    cudaError_t ensure_side(bool high) {
+        int least = 0, greatest = 0;
+        cudaError_t e = cudaDeviceGetStreamPriorityRange(&least, &greatest);
+        for (int k = 0; k < (high ? 2 : 1) && e == cudaSuccess; ++k)
+            if (!side[k]) e = cudaStreamCreateWithPriority(&side[k], cudaStreamNonBlocking, k ? greatest : least);
+        if (e == cudaSuccess && !fork) e = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
+        if (e == cudaSuccess && !join) e = cudaEventCreateWithFlags(&join, cudaEventDisableTiming);
+        return e;
+    }
+
     cenote_stats stats{};
     unsigned long long tally_prev[6] = {0, 0, 0, 0, 0, 0};
 
     ~cenote_renderer() {
         for (cudaEvent_t e : events) cudaEventDestroy(e);
+        for (cudaStream_t s : side)
+            if (s) cudaStreamDestroy(s);
+        if (fork) cudaEventDestroy(fork);
+        if (join) cudaEventDestroy(join);
     }
     cudaEvent_t event(size_t i) {
         while (events.size() <= i) {

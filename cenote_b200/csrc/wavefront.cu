@@ -59,6 +59,23 @@ constexpr int BLOCK = 128;
 
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31u; }
 
+// How a persistent grid shares `count` items: every warp owns a first batch of
+// `quota` items at a place known from its index, and the rest go out in
+// batches of up to 32 from a counter. A queue that the first batches cover
+// costs no atomics at all (thousands of warps asking one address for nothing
+// took longer than the late bounces' work), and below 32 items a warp it is
+// spread over more warps, at least `least` to a warp: fewer divergent items
+// share a warp and more warps hide each other's latency.
+struct WarpShare {
+    uint32_t first, quota, rest;  // this warp's first item, its items, the first item off the counter
+};
+__device__ __forceinline__ WarpShare warp_share(uint32_t count, uint32_t least) {
+    const uint32_t per_block = blockDim.x >> 5, warps = gridDim.x * per_block;
+    const uint32_t w = blockIdx.x * per_block + (threadIdx.x >> 5);
+    const uint32_t quota = min(32u, max(least, (count + warps - 1u) / warps));
+    return {w * quota, quota, warps * quota};
+}
+
 // Fetch the next 32 work items for this warp; every lane gets the same base.
 __device__ __forceinline__ uint32_t warp_fetch(uint32_t* counter) {
     uint32_t base = 0;
@@ -227,14 +244,38 @@ __global__ void __launch_bounds__(BLOCK) k_raygen_segments(PathPool pool, const 
 
 __device__ __forceinline__ uint32_t lanemask_lt() { return (1u << lane_id()) - 1u; }
 
+// The least items of a spread queue's warps (warp_share). Device time of a
+// one-sample 640x360 chart frame and a two-sample 853x479 terrain frame at 32,
+// 16, 8, 4 and 1 for the walks and 8 for shading: 1.04, 1.02, 1.04, 1.06, 1.08
+// and 3.71, 3.66, 3.62, 3.62, 3.77 ms: a step of a walk costs a warp the same
+// for 8 rays as for 32, so fewer rays a warp only pay while warps lack.
+// Shading at 1 instead of 8: 1.00 and 3.53 ms (a warp there runs every branch
+// its items take). Waves of millions of paths are level at any value.
+#ifndef CN_QUOTA_TRAV
+#define CN_QUOTA_TRAV 8
+#endif
+#ifndef CN_QUOTA_SHADE
+#define CN_QUOTA_SHADE 1
+#endif
+
 // Hand the warp's idle lanes their next work items: returns this lane's item
 // index (or ~0u) and sets `drained` (warp-uniform) once the queue is used up.
-__device__ __forceinline__ uint32_t refill(uint32_t* counter, uint32_t count, bool live, bool& drained) {
+// `rest` is 0 before the warp's first batch (warp_share) and the first item
+// off the counter after it.
+__device__ __forceinline__ uint32_t refill(uint32_t* counter, uint32_t count, bool live, bool& drained,
+                                           uint32_t& rest) {
+    if (rest == 0u) {
+        const WarpShare ws = warp_share(count, CN_QUOTA_TRAV);
+        rest = ws.rest;
+        drained = rest >= count;
+        const uint32_t i = ws.first + lane_id();
+        return lane_id() < ws.quota && i < count ? i : ~0u;
+    }
     uint32_t idle = __ballot_sync(0xffffffffu, !live);
     if (idle == 0) return ~0u;
     uint32_t base = 0;
     if (lane_id() == 0) base = atomicAdd(counter, uint32_t(__popc(idle)));
-    base = __shfl_sync(0xffffffffu, base, 0);
+    base = rest + __shfl_sync(0xffffffffu, base, 0);
     if (base + uint32_t(__popc(idle)) >= count) drained = true;
     if (live) return ~0u;
     uint32_t i = base + __popc(idle & lanemask_lt());
@@ -261,6 +302,7 @@ __global__ void __launch_bounds__(B, CN_ISECT_MIN_BLOCKS * BLOCK / B)
     Ray ray;
     float tmax = 1e30f, best_b1 = 0.0f, best_b2 = 0.0f;
     uint32_t path = 0, best_inst = LIGHT_NONE, best_prim = 0, crossings = 0, pixel = 0, sample = 0;
+    uint32_t rest = 0;        // refill's state
     uint32_t qi = 0;          // the ray's queue position (the material sort's key slot)
     bool live = false, drained = false, finished = false;
     // The rays that finished since the last refill: their hits and, when this
@@ -306,7 +348,7 @@ __global__ void __launch_bounds__(B, CN_ISECT_MIN_BLOCKS * BLOCK / B)
     for (;;) {
         retire();
         if (!drained) {
-            uint32_t i = refill(fetch, count, live, drained);
+            uint32_t i = refill(fetch, count, live, drained, rest);
             if (i != ~0u) {
                 qi = i;
                 path = bounce == 0 ? i : queue[i];
@@ -362,8 +404,11 @@ struct IsectSource {
     const uint32_t* queue;
     uint32_t* fetch;
     uint32_t count, bounce;
+    uint32_t rest = 0;
     __device__ __forceinline__ uint32_t path_of(uint32_t i) const { return bounce == 0 ? i : queue[i]; }
-    __device__ __forceinline__ uint32_t next(bool live, bool& drained) { return refill(fetch, count, live, drained); }
+    __device__ __forceinline__ uint32_t next(bool live, bool& drained) {
+        return refill(fetch, count, live, drained, rest);
+    }
     __device__ __forceinline__ void ray(uint32_t i, float3& o, float3& d) const {
         const uint32_t path = path_of(i);
         o = xyz(pool.org[path]);
@@ -506,14 +551,15 @@ __global__ void __launch_bounds__(BLOCK, LAYERS ? CN_SHADE_LAYERED_MIN_BLOCKS : 
     const uint32_t* queue = pool.queue[bounce & 1u];
     uint32_t* next_queue = pool.queue[(bounce + 1u) & 1u];
     uint32_t* fetch = pool.counters + (part == 2 ? CTR_FETCH_SHADE_LAYERS : CTR_FETCH_SHADE) + bounce;
+    const WarpShare ws = warp_share(count - min(first, count), CN_QUOTA_SHADE);
+    uint32_t base = first + ws.first, quota = ws.quota;
     for (;;) {
-        uint32_t base = first + warp_fetch(fetch);
         if (base >= count) break;
         uint32_t i = base + lane_id();
         bool push_ray = false, push_shadow = false;
         uint32_t path = 0;
         ShadowRay sr;
-        if (i < count) {
+        if (i < count && lane_id() < quota) {
             path = pool.order ? pool.order[i] : (bounce == 0 ? i : queue[i]);
             uint4 h = pool.hit[path];
             float4 d4 = pool.dir[path];
@@ -777,6 +823,9 @@ __global__ void __launch_bounds__(BLOCK, LAYERS ? CN_SHADE_LAYERED_MIN_BLOCKS : 
                 flag_overflow(pool.counters);
             }
         }
+        if (first + ws.rest >= count) break;
+        base = first + ws.rest + warp_fetch(fetch);
+        quota = 32u;
     }
 }
 
@@ -794,11 +843,11 @@ __global__ void __launch_bounds__(B, CN_TRAV_MIN_BLOCKS * BLOCK / B)
     ShadowQuery q;
     Ray ray;
     float3 contrib = f3(0.0f);
-    uint32_t path = 0;
+    uint32_t path = 0, rest = 0;
     bool live = false, drained = false;
     for (;;) {
         if (!drained) {
-            uint32_t i = refill(fetch, count, live, drained);
+            uint32_t i = refill(fetch, count, live, drained, rest);
             if (i != ~0u) {
                 const float4* rec = reinterpret_cast<const float4*>(pool.shadows + i);
                 float4 q0 = rec[0], q1 = rec[1], q2 = rec[2], q3 = rec[3];
@@ -847,7 +896,10 @@ struct ShadowSource {
     const PathPool& pool;
     uint32_t* fetch;
     uint32_t count;
-    __device__ __forceinline__ uint32_t next(bool live, bool& drained) { return refill(fetch, count, live, drained); }
+    uint32_t rest = 0;
+    __device__ __forceinline__ uint32_t next(bool live, bool& drained) {
+        return refill(fetch, count, live, drained, rest);
+    }
     __device__ __forceinline__ bool begin(uint32_t i, Ray& ray, AnyQuery& a) const {
         const float4* rec = reinterpret_cast<const float4*>(pool.shadows + i);
         const float4 q0 = rec[0], q1 = rec[1], q2 = rec[2], q3 = rec[3];
