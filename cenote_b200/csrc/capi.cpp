@@ -697,6 +697,21 @@ int32_t cenote_scene_create_textured(cenote_context* ctx, const cenote_object* o
                                 ctx->stream));
     CN_CUDA(cudaStreamSynchronize(ctx->stream));
 
+    auto closure_class = [](const Material& m) {
+        return (m.specular_weight != 0.0f ? 1u : 0u) | (m.metalness != 0.0f ? 2u : 0u);
+    };
+    uint32_t classes = 0;  // of the materials that reflect
+    bool maps = false;
+    for (const Material& m : mats) {
+        maps = maps || (m.base_color_texture & m.specular_roughness_texture & m.metalness_texture & m.emission_texture &
+                        m.opacity_texture & m.normal_texture) != TEXTURE_NONE;
+        const bool dark = m.specular_weight == 0.0f && m.base_color[0] == 0.0f && m.base_color[1] == 0.0f &&
+                          m.base_color[2] == 0.0f;
+        if (!dark) classes |= 1u << closure_class(m);
+    }
+    sc->uniform_shading = !maps && !layered && (classes & (classes - 1u)) == 0u &&
+                          tri_count <= cenote_renderer::UNIFORM_MAX_TRIANGLES;
+
     DeviceScene& ds = sc->ds;
     ds.textures = btexs->as<unsigned long long>();
     ds.texture_count = texture_count;
@@ -875,6 +890,7 @@ int32_t cenote_renderer_set_material_sort(cenote_renderer* r, uint32_t mode) {
     CN_CHECK(r, CENOTE_E_INVALID_ARGUMENT, "null renderer");
     CN_CHECK(mode <= CENOTE_SORT_SECONDARY, CENOTE_E_INVALID_ARGUMENT, "unknown material-sort mode");
     r->material_sort = mode;
+    r->sort_chosen = true;
     return CENOTE_OK;
 }
 
@@ -896,6 +912,7 @@ int32_t cenote_renderer_set_tuning(cenote_renderer* r, const cenote_tuning* t) {
              "stack_depth is 16 or 32");
     CN_CHECK(t->sort_by_location <= 1, CENOTE_E_INVALID_ARGUMENT, "sort_by_location is 0 or 1");
     r->material_sort = t->material_sort;
+    r->sort_chosen = true;
     r->samples_per_wave = t->samples_per_wave;
     r->refill_idle = t->refill_idle;
     r->top_nodes = t->top_nodes;
@@ -1053,7 +1070,7 @@ int32_t run_waves(cenote_renderer* r, cenote_scene* sc, uint32_t width, uint32_t
     WavePlan plan = plan_waves(r, pixels, count, oneshot != nullptr);
     CN_CHECK(plan.need < (1ull << 31), CENOTE_E_INVALID_ARGUMENT, "wave too large");
     CN_CUDA(r->ensure(plan.need));
-    CN_CUDA(r->ensure_side(false));
+    CN_CUDA(r->ensure_side());
     // Films trace the guides (Renderer::accumulate); one-shot renders do not.
     CN_CUDA(r->set_guides(film != nullptr));
     CN_CUDA(r->set_learned_guide(r->guide != nullptr));
@@ -1146,6 +1163,7 @@ int32_t cenote_renderer_autotune(cenote_renderer* r, cenote_scene* scene, uint32
                        r->sort_by_location};
     auto apply = [&](const cenote_tuning& t) {
         r->material_sort = t.material_sort;
+        r->sort_chosen = true;
         r->samples_per_wave = t.samples_per_wave;
         r->refill_idle = t.refill_idle;
         r->top_nodes = t.top_nodes;

@@ -78,24 +78,21 @@ WavePlan plan_waves(const cenote_renderer* r, uint64_t pixels, uint32_t count, b
 
 // The bounces of one wave of n0 camera paths already in the pool: per
 // bounce intersect, (the guide's inference,) the material sort, shade and
-// shadow. A bounce's shadow walk runs on the renderer's side stream beside the
-// next bounce's intersect and sort, which touch nothing it reads or writes
+// shadow. With a `side` stream of its own a bounce's shadow walk runs beside
+// the next bounce's intersect and sort, which touch nothing it reads or writes
 // (it adds to the radiance that the next shade reads): the two walks fill
 // each other's tails, and on small waves the shorter one's latency vanishes.
-// Timing marks bracket intersect, shade and shadow when `timing`, which keeps
-// them in turn on one stream.
+// Timing marks bracket intersect, shade and shadow when `timing`: the caller
+// then keeps them in turn on one stream.
 void enqueue_bounces(cenote_renderer* r, const cenote_scene* sc, const WaveParams& wp, uint32_t n0, bool guided,
-                     cudaStream_t stream, bool timing, bool counting, WaveCounts* wc) {
+                     cudaStream_t stream, cudaStream_t side, bool timing, bool counting, WaveCounts* wc) {
     cenote_context* ctx = r->ctx;
     auto mark = [&]() {
         if (timing) cudaEventRecord(r->event(wc->events++), stream);
     };
-    int priority = 0, least = 0, greatest = 0;
-    cudaDeviceGetStreamPriorityRange(&least, &greatest);
-    cudaStreamGetPriority(stream, &priority);
-    cudaStream_t side = timing ? stream : r->side[priority < least ? 1 : 0];
+    const uint32_t mode = r->sort_mode(sc, n0);
     for (uint32_t b = 0; b < wp.max_bounces; ++b) {
-        const bool sort = r->material_sort == CENOTE_SORT_ALL || (r->material_sort == CENOTE_SORT_SECONDARY && b > 0);
+        const bool sort = mode == CENOTE_SORT_ALL || (mode == CENOTE_SORT_SECONDARY && b > 0);
         const PathPool view = sort ? r->sorted_view() : r->pool;
         if (sort) launch_sort_begin(view, stream);
         launch_intersect(sc->ds, view, b, n0, ctx->shape, counting, stream);
@@ -146,7 +143,10 @@ cudaError_t enqueue_segments(cenote_renderer* r, const cenote_scene* sc, const W
     wp.light_sampling = r->light_sampling;
     const uint32_t n0 = hdr ? 0u : paths;  // 0: the kernels read the count raygen leaves
     launch_wave_begin_segments(r->pool, segs, nseg, paths, hdr, r->ctx->shape, stream);
-    enqueue_bounces(r, sc, wp, n0, false, stream, false, false, wc);
+    // One stream: two lanes of waves overlap as it is, and a forked graph
+    // takes longer to instantiate and launch (twelve small jobs 15.4 against
+    // 14.6 ms).
+    enqueue_bounces(r, sc, wp, n0, false, stream, stream, false, false, wc);
     launch_tally(r->pool, r->tally.as<unsigned long long>(), n0, max_bounces, stream);
     launch_accumulate_segments(r->pool, segs, nseg, items, hdr, stream);
     wc->launches += 2 + 3 * max_bounces;
@@ -209,7 +209,7 @@ cudaError_t enqueue_waves(cenote_renderer* r, const cenote_scene* sc, uint32_t w
             if (guided) cudaMemsetAsync(r->g_count.ptr, 0, 4, stream);
             launch_wave_begin(r->pool, wp, ctx->shape, stream);
             mark();
-            enqueue_bounces(r, sc, wp, n0, guided, stream, timing, counting, wc);
+            enqueue_bounces(r, sc, wp, n0, guided, stream, timing ? stream : r->side, timing, counting, wc);
             launch_tally(r->pool, r->tally.as<unsigned long long>(), n0, max_bounces, stream);
             if (film)
                 launch_accumulate(r->pool, *film, wp.pixel_base, wp.pixel_count, wp.tile_width, s,

@@ -108,6 +108,10 @@ struct cenote_scene {
     float select_prob = 0.0f;
     float prep_ms[3] = {0, 0, 0};
     uint32_t bvh_builder = CENOTE_BVH_HOST_SAH;  // the builder this scene's BVH came from
+    // Every material runs the same closure code (no maps, no layers, specular
+    // and metal on all or on none) and the geometry is small: a material sort
+    // has nothing to group.
+    bool uniform_shading = false;
     uint64_t device_bytes = 0;
     DeviceBuffer* env_marginal = nullptr;
     DeviceBuffer* env_conditional = nullptr;
@@ -152,6 +156,7 @@ struct cenote_renderer {
     // (every bounce by default: 1.1x on the material chart, 1.6x on the
     // textured 2 M-triangle terrain, measured on a B200).
     uint32_t material_sort = 1;
+    bool sort_chosen = false;  // set by the caller or the autotuner: then it holds for every wave
     uint32_t refill_idle = 0;  // 0: the kernels' default
     uint32_t top_nodes = 0;    // BVH nodes staged in shared memory by the traversal kernels
     uint32_t l2_window = 0;    // mark the BVH nodes persisting in L2 during this renderer's waves
@@ -171,16 +176,14 @@ struct cenote_renderer {
     size_t g_cap = 0;
     static constexpr uint32_t GUIDE_RECORDS = 1u << 20;
     static constexpr uint32_t GUIDE_BATCH = 65536;
-    // The shadow walks' own stream (index 1: at the highest priority, beside a
-    // main stream of that priority) and the events that fork it off the main
-    // stream and join it back, every bounce of every wave.
-    cudaStream_t side[2] = {nullptr, nullptr};
+    // The shadow walks' own stream and the events that fork it off the main
+    // stream and join it back, every bounce of every wave (made on the first
+    // wave; serving waves do without).
+    cudaStream_t side = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
-    cudaError_t ensure_side(bool high) {
-        int least = 0, greatest = 0;
-        cudaError_t e = cudaDeviceGetStreamPriorityRange(&least, &greatest);
-        for (int k = 0; k < (high ? 2 : 1) && e == cudaSuccess; ++k)
-            if (!side[k]) e = cudaStreamCreateWithPriority(&side[k], cudaStreamNonBlocking, k ? greatest : least);
+    cudaError_t ensure_side() {
+        cudaError_t e = cudaSuccess;
+        if (!side) e = cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking);
         if (e == cudaSuccess && !fork) e = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
         if (e == cudaSuccess && !join) e = cudaEventCreateWithFlags(&join, cudaEventDisableTiming);
         return e;
@@ -191,8 +194,7 @@ struct cenote_renderer {
 
     ~cenote_renderer() {
         for (cudaEvent_t e : events) cudaEventDestroy(e);
-        for (cudaStream_t s : side)
-            if (s) cudaStreamDestroy(s);
+        if (side) cudaStreamDestroy(side);
         if (fork) cudaEventDestroy(fork);
         if (join) cudaEventDestroy(join);
     }
@@ -203,6 +205,23 @@ struct cenote_renderer {
             events.push_back(e);
         }
         return events[i];
+    }
+
+    // The sort mode of a wave of `paths` camera paths (0: known on the device
+    // only). Unless a mode was chosen, waves whose bounces shade no faster in
+    // material order skip it; films are the same bits either way where the
+    // scene has no layered materials (with them, the sorted bounces split
+    // between two builds of the shading kernel). Measured device ms, sorted /
+    // unsorted: one closure class, 1 M paths, 36 to 20,412 triangles 1.58 /
+    // 1.43 to 2.87 / 2.67, 7.4 M paths 6.04 / 5.30 to 10.3 / 9.2; the chart at
+    // 0.23 M paths 1.00 / 0.91, at 0.92 M 1.69 / 1.75, at 16.6 M 16.7 / 19.4;
+    // the textured scene at 0.23 M 0.36 / 0.33, at 0.92 M 0.72 / 1.01.
+    static constexpr uint32_t SORT_MIN_PATHS = 1u << 18;
+    static constexpr uint32_t UNIFORM_MAX_TRIANGLES = 1u << 15;
+    uint32_t sort_mode(const cenote_scene* sc, uint32_t paths) const {
+        if (sort_chosen || sc->ds.has_layers) return material_sort;
+        if (sc->uniform_shading || (paths != 0 && paths < SORT_MIN_PATHS)) return CENOTE_SORT_NONE;
+        return material_sort;
     }
 
     cudaError_t ensure(size_t cap) {
@@ -364,9 +383,10 @@ cudaError_t enqueue_waves(cenote_renderer* r, const cenote_scene* sc, uint32_t w
                           const FilmTargets* film, bool film_reset, float4* oneshot, const uint32_t* sample_offset,
                           cudaStream_t stream, bool timing, bool counting, WaveCounts* wc);
 
-// The bounces of one wave whose n0 camera paths are in the pool.
+// The bounces of one wave whose n0 camera paths are in the pool; `side` may be
+// `stream`.
 void enqueue_bounces(cenote_renderer* r, const cenote_scene* sc, const WaveParams& wp, uint32_t n0, bool guided,
-                     cudaStream_t stream, bool timing, bool counting, WaveCounts* wc);
+                     cudaStream_t stream, cudaStream_t side, bool timing, bool counting, WaveCounts* wc);
 
 // One multi-job wave (the serving loop): segments in device memory, their
 // camera paths, the bounces, and each segment's samples into its job's film.

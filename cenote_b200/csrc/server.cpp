@@ -672,7 +672,6 @@ int32_t cenote_server_create(cenote_context* ctx, uint64_t hbm_budget, const cen
         cenote_renderer& r = s->renderers[k];
         r.ctx = ctx;
         r.light_sampling = s->opt.light_sampling;
-        CN_CUDA(r.ensure_side(true));
         CN_CUDA(r.ensure(s->opt.pool_paths));
         CN_CUDA(r.counters.alloc(CTR_COUNT * 4));
         CN_CUDA(r.tally.alloc(64));

@@ -282,7 +282,9 @@ int32_t cenote_renderer_stats(cenote_renderer* r, cenote_stats* out);
 #define CENOTE_SORT_NONE 0u
 #define CENOTE_SORT_ALL 1u
 #define CENOTE_SORT_SECONDARY 2u /* every bounce but the camera rays' */
-/* A new renderer sorts every bounce (CENOTE_SORT_ALL). */
+/* A new renderer sorts every bounce (CENOTE_SORT_ALL) of the waves that gain
+ * by it: small ones and scenes of one kind of material skip the sort, with the
+ * same film. A mode set here holds for every wave. */
 int32_t cenote_renderer_set_material_sort(cenote_renderer* r, uint32_t mode);
 /* The per-scene launch knobs. None changes a result: every setting renders
  * the same film bit for bit. */
