@@ -590,7 +590,7 @@ __global__ void __launch_bounds__(TILE * WG, 1) k_infer_paths(Net net, DeviceSce
             const uint4 h = pool.hit[path];
             hit = h.x != LIGHT_NONE;
             if (hit) {
-                const float4 d4 = pool.dir[path];
+                const float4 d4 = pool.dir(path);
                 const float3 dir = make_float3(d4.x, d4.y, d4.z);
                 float3 wp;
                 hit_frame(scene, h, dir, wp, nrm);
@@ -662,13 +662,13 @@ __global__ void __launch_bounds__(TILE * WG, 1) k_infer_paths(Net net, DeviceSce
 
 __device__ __forceinline__ float lum(float3 c) { return 0.2722287f * c.x + 0.6740818f * c.y + 0.0536895f * c.z; }
 
-__global__ void k_resolve_records(Record* recs, const uint32_t* count, uint32_t capacity, const float4* rad) {
+__global__ void k_resolve_records(Record* recs, const uint32_t* count, uint32_t capacity, const float4* flux) {
     const uint32_t n = min(*count, capacity);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         Record r = recs[i];
         float c = 0.0f;
         if (r.q2.w >= 0.0f && r.q0.w > 0.0f) {
-            float4 f = rad[__float_as_uint(r.q3.w)];
+            float4 f = flux[2 * size_t(__float_as_uint(r.q3.w)) + 1];  // the path's radiance
             float L = (lum(make_float3(f.x, f.y, f.z)) - r.q2.w) / fmaxf(r.q1.w, 1e-12f);
             c = fmaxf(L, 0.0f) / r.q0.w;
             if (!isfinite(c)) c = 0.0f;
@@ -831,8 +831,8 @@ void launch_infer_paths(const Buffers& b, const DeviceScene& scene, const PathPo
     k_infer_paths<<<sms, TILE * WG, InferSmem::BYTES, s>>>(view(b), scene, pool, bounce, n0, b.err);
 }
 
-void launch_resolve_records(Record* recs, const uint32_t* count, uint32_t capacity, const float4* rad, cudaStream_t s) {
-    k_resolve_records<<<148 * 4, 256, 0, s>>>(recs, count, capacity, rad);
+void launch_resolve_records(Record* recs, const uint32_t* count, uint32_t capacity, const float4* flux, cudaStream_t s) {
+    k_resolve_records<<<148 * 4, 256, 0, s>>>(recs, count, capacity, flux);
 }
 
 void launch_train_records(const Buffers& b, const TrainScratch& t, const Record* recs, const uint32_t* count,

@@ -215,7 +215,7 @@ void launch_infer_paths(const Buffers& b, const DeviceScene& scene, const PathPo
                         uint32_t n0, int sms, cudaStream_t s);
 // Turn the wave's records into target weights L / pdf (L from the paths'
 // final radiance and the snapshot the next vertex took).
-void launch_resolve_records(Record* recs, const uint32_t* count, uint32_t capacity, const float4* rad, cudaStream_t s);
+void launch_resolve_records(Record* recs, const uint32_t* count, uint32_t capacity, const float4* flux, cudaStream_t s);
 
 // Scratch of the training steps (device).
 struct TrainScratch {

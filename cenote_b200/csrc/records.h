@@ -136,17 +136,17 @@ struct DeviceScene {
     uint32_t top_smem;
 };
 
-// One queued shadow ray: 64 bytes, four 16-byte lanes.
+// One shadow ray: 64 bytes, four 16-byte lanes (two whole sectors).
 struct alignas(16) ShadowRay {
     float org[3];
     float tmax;
     float dir[3];
-    uint32_t path;
+    uint32_t pad;
     float contrib[3];
     uint32_t light;
     uint32_t primitive;
     uint32_t leaf;     // the target triangle's leaf index, ~0 when unknown or none
-    uint32_t pad[2];
+    uint32_t pad1[2];
 };
 
 }  // namespace cn

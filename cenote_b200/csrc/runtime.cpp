@@ -220,7 +220,7 @@ cudaError_t enqueue_waves(cenote_renderer* r, const cenote_scene* sc, uint32_t w
             if (guided) {
                 guide::Record* recs = r->g_records.as<guide::Record>();
                 const uint32_t* cnt = r->g_count.as<uint32_t>();
-                guide::launch_resolve_records(recs, cnt, cenote_renderer::GUIDE_RECORDS, r->pool.rad, stream);
+                guide::launch_resolve_records(recs, cnt, cenote_renderer::GUIDE_RECORDS, r->pool.flux, stream);
                 const float3 bmin = make_float3(sc->ds.bbox_min[0], sc->ds.bbox_min[1], sc->ds.bbox_min[2]);
                 for (uint32_t k = 0; k < r->guide_steps; ++k) {
                     r->guide->step++;

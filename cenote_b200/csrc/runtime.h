@@ -151,7 +151,7 @@ struct cenote_renderer {
     uint32_t profiling = 0;
     std::vector<cudaEvent_t> events;
     PathPool pool{};
-    DeviceBuffer org, dir, thr, hit, ps, state, rad, q0, q1, shadows, counters, tally, scratch;
+    DeviceBuffer ray, flux, hit, ps, q0, q1, shadows, shadow_queue, counters, tally, scratch;
     // Material sort before shading: CENOTE_SORT_NONE, _ALL or _SECONDARY
     // (every bounce by default: 1.1x on the material chart, 1.6x on the
     // textured 2 M-triangle terrain, measured on a B200).
@@ -165,7 +165,7 @@ struct cenote_renderer {
     uint32_t sort_by_location = 0;    // 1: the material sort keys layer-free hits by location
     float tuned_ms_per_sample = 0.0f;
     DeviceBuffer sort_order, sort_keys, sort_bins;
-    DeviceBuffer aov_albedo, aov_normal, aov_depth, aov_guide;
+    DeviceBuffer aov, aov_guide;
     size_t pool_cap = 0, aov_cap = 0;
     // The learned guide (cenote_renderer_set_guide): per-path mixture outputs
     // and open records, the wave's training records and its sink.
@@ -227,22 +227,19 @@ struct cenote_renderer {
     cudaError_t ensure(size_t cap) {
         if (cap <= pool_cap) return cudaSuccess;
         cudaError_t e;
-        if ((e = org.alloc(cap * 16)) || (e = dir.alloc(cap * 16)) || (e = thr.alloc(cap * 16)) ||
-            (e = hit.alloc(cap * 16)) || (e = ps.alloc(cap * 8)) || (e = state.alloc(cap * 4)) ||
-            (e = rad.alloc(cap * 16)) || (e = q0.alloc(cap * 4)) || (e = q1.alloc(cap * 4)) ||
-            (e = shadows.alloc(cap * sizeof(ShadowRay))) || (e = sort_order.alloc(cap * 4)) ||
+        if ((e = ray.alloc(cap * 32)) || (e = flux.alloc(cap * 32)) || (e = hit.alloc(cap * 16)) ||
+            (e = ps.alloc(cap * 8)) || (e = q0.alloc(cap * 4)) || (e = q1.alloc(cap * 4)) ||
+            (e = shadows.alloc(cap * sizeof(ShadowRay))) || (e = shadow_queue.alloc(cap * 4)) || (e = sort_order.alloc(cap * 4)) ||
             (e = sort_keys.alloc(cap * 4)) || (e = sort_bins.alloc(cn::SORT_BINS * 4)))
             return e;
-        pool.org = org.as<float4>();
-        pool.dir = dir.as<float4>();
-        pool.thr = thr.as<float4>();
+        pool.ray = ray.as<float4>();
+        pool.flux = flux.as<float4>();
         pool.hit = hit.as<uint4>();
         pool.ps = ps.as<uint2>();
-        pool.state = state.as<uint32_t>();
-        pool.rad = rad.as<float4>();
         pool.queue[0] = q0.as<uint32_t>();
         pool.queue[1] = q1.as<uint32_t>();
         pool.shadows = shadows.as<ShadowRay>();
+        pool.shadow_queue = shadow_queue.as<uint32_t>();
         // Null here: the wave loop passes a view with all three set to the
         // bounces it sorts.
         pool.order = nullptr;
@@ -286,14 +283,10 @@ struct cenote_renderer {
         cudaError_t set_guides(bool on) {
         if (on && aov_cap < pool_cap) {
             cudaError_t e;
-            if ((e = aov_albedo.alloc(pool_cap * 16)) || (e = aov_normal.alloc(pool_cap * 16)) ||
-                (e = aov_depth.alloc(pool_cap * 4)) || (e = aov_guide.alloc(pool_cap * 16)))
-                return e;
+            if ((e = aov.alloc(pool_cap * 32)) || (e = aov_guide.alloc(pool_cap * 16))) return e;
             aov_cap = pool_cap;
         }
-        pool.aov_albedo = on ? aov_albedo.as<float4>() : nullptr;
-        pool.aov_normal = on ? aov_normal.as<float4>() : nullptr;
-        pool.aov_depth = on ? aov_depth.as<float>() : nullptr;
+        pool.aov = on ? aov.as<float4>() : nullptr;
         pool.aov_guide = on ? aov_guide.as<float4>() : nullptr;
         return cudaSuccess;
     }

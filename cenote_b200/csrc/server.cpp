@@ -200,7 +200,7 @@ struct cenote_server {
     std::map<uint64_t, std::unique_ptr<float[]>> results;
 
     static uint64_t job_bytes(uint32_t w, uint32_t h) { return uint64_t(w) * h * 32; }
-    static uint64_t path_bytes() { return 16 * 5 + 8 + 4 + 8 + sizeof(ShadowRay) + 8; }
+    static uint64_t path_bytes() { return 32 * 2 + 16 + 8 + 8 + sizeof(ShadowRay) + 4 + 8; }
 
     cudaError_t take_dev(DeviceBuffer& b, size_t bytes) {
         auto it = free_dev.find(bytes);

@@ -34,17 +34,16 @@ namespace {
 constexpr int BLOCK = 128;
 
 // Minimum resident 128-thread blocks per SM for the shading kernel: the
-// register cap that trades spills against occupancy (6 → 80 registers; with
-// material-sorted waves of 30-60 M paths, 6 measured 2 % faster than 5 on the
-// textured terrain and level on the chart; 4 and uncapped were slower).
+// register cap that trades spills against occupancy. 7 (72 registers, 118 /
+// 288 bytes of spills per thread) shades the chart in 25.2 ms per frame and
+// the terrain in 84.2 against 25.9 and 84.3 at 6 (80 registers); 5 measured
+// 27.3 and 85.9, 8 (64 registers) 25.9 and 85.7.
 #ifndef CN_SHADE_MIN_BLOCKS
-#define CN_SHADE_MIN_BLOCKS 6
+#define CN_SHADE_MIN_BLOCKS 7
 #endif
 // The same for the variant with the coat, fuzz, transmission and thin-wall
 // lobes, which needs more registers than the layer-free one: 4 (128
-// registers, 82 / 152 bytes of spills per thread instead of 374 / 908 at 80)
-// shades the terrain in 86.2 ms per frame against 87.2 at 6 and 89.0 at 5
-// (two runs each); the layer-free variant keeps 6.
+// registers, no spills) and 5 (96) are level on the terrain, 6 slower.
 #ifndef CN_SHADE_LAYERED_MIN_BLOCKS
 #define CN_SHADE_LAYERED_MIN_BLOCKS 4
 #endif
@@ -83,16 +82,17 @@ __device__ __forceinline__ uint32_t warp_fetch(uint32_t* counter) {
     return __shfl_sync(0xffffffffu, base, 0);
 }
 
-// Warp-aggregated append: returns this lane's slot, or ~0u if !pred. Must be
-// called by all 32 lanes together.
-__device__ __forceinline__ uint32_t warp_push(uint32_t* counter, bool pred) {
-    uint32_t mask = __ballot_sync(0xffffffffu, pred);
-    if (mask == 0) return ~0u;
-    uint32_t leader = __ffs(mask) - 1u;
+// Warp-aggregated appends to two queues: this lane's slots in each, or ~0u
+// where its predicate is false. One atomic per queue and warp, both issued by
+// the same instruction. Must be called by all 32 lanes together.
+__device__ __forceinline__ uint2 warp_push2(uint32_t* ca, bool pa, uint32_t* cb, bool pb) {
+    const uint32_t ma = __ballot_sync(0xffffffffu, pa), mb = __ballot_sync(0xffffffffu, pb);
     uint32_t base = 0;
-    if (lane_id() == leader) base = atomicAdd(counter, uint32_t(__popc(mask)));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    return pred ? base + __popc(mask & ((1u << lane_id()) - 1u)) : ~0u;
+    const uint32_t n = __popc(lane_id() == 0 ? ma : mb);
+    if (lane_id() < 2u && n) base = atomicAdd(lane_id() == 0 ? ca : cb, n);
+    const uint32_t below = (1u << lane_id()) - 1u;
+    const uint32_t a = __shfl_sync(0xffffffffu, base, 0), b = __shfl_sync(0xffffffffu, base, 1);
+    return make_uint2(pa ? a + __popc(ma & below) : ~0u, pb ? b + __popc(mb & below) : ~0u);
 }
 
 __device__ __forceinline__ void flag_overflow(uint32_t* counters) { atomicOr(counters + CTR_OVERFLOW, 1u); }
@@ -108,7 +108,8 @@ __device__ __forceinline__ uint32_t material_key(const DeviceScene& s, const Pat
     if (inst == LIGHT_NONE) return 0u;
     if (__ldg(s.instance_layers + inst)) return SORT_LAYERS + inst % (SORT_BINS - SORT_LAYERS);
     if (!pool.sort_location) return 1u + inst % (SORT_LAYERS - 1u);
-    const float4 o = pool.org[path], d = pool.dir[path];
+    const Float4Pair ray = load_pair(&pool.org(path));
+    const float4 o = ray.a, d = ray.b;
     const float fx = (o.x + t * d.x - s.bbox_min[0]) * s.bbox_inv, fz = (o.z + t * d.z - s.bbox_min[2]) * s.bbox_inv;
     const uint32_t cx = min(31u, uint32_t(fmaxf(fx, 0.0f) * 32.0f)), cz = min(31u, uint32_t(fmaxf(fz, 0.0f) * 32.0f));
     uint32_t m = 0u;
@@ -173,17 +174,14 @@ __device__ __forceinline__ void raygen_path(const PathPool& pool, uint32_t p, ui
         org = org + off;
         dir = normalize(target - off);
     }
-    pool.org[p] = f4(org, 0.0f);
-    pool.dir[p] = f4(dir, dot(dir, normalize(cam_fwd)));
-    pool.thr[p] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
+    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    store_pair(&pool.org(p), f4(org, __uint_as_float(MEDIUM_NONE)), f4(dir, dot(dir, normalize(cam_fwd))));
+    store_pair(&pool.thr(p), make_float4(1.0f, 1.0f, 1.0f, 0.0f), zero);
     pool.ps[p] = make_uint2(pixel, sample);
-    pool.state[p] = MEDIUM_NONE;
-    pool.rad[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if (pool.guide_rec) pool.guide_rec[p] = ~0u;
-    if (pool.aov_albedo) {
-        pool.aov_albedo[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        pool.aov_normal[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        pool.aov_depth[p] = 0.0f;
+    if (pool.aov) {
+        store_pair(&pool.albedo(p), zero, zero);
+        pool.aov_guide[p] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
     }
 }
 
@@ -352,8 +350,8 @@ __global__ void __launch_bounds__(B, CN_ISECT_MIN_BLOCKS * BLOCK / B)
             if (i != ~0u) {
                 qi = i;
                 path = bounce == 0 ? i : queue[i];
-                float4 o = pool.org[path], d = pool.dir[path];
-                ray = make_ray(xyz(o), xyz(d));
+                const Float4Pair od = load_pair(&pool.org(path));
+                ray = make_ray(xyz(od.a), xyz(od.b));
                 tmax = 1e30f;
                 best_inst = LIGHT_NONE;
                 best_prim = 0;
@@ -411,8 +409,9 @@ struct IsectSource {
     }
     __device__ __forceinline__ void ray(uint32_t i, float3& o, float3& d) const {
         const uint32_t path = path_of(i);
-        o = xyz(pool.org[path]);
-        d = xyz(pool.dir[path]);
+        const Float4Pair od = load_pair(&pool.org(path));
+        o = xyz(od.a);
+        d = xyz(od.b);
     }
     __device__ __forceinline__ void emit(uint32_t i, uint4 hit, float) const { pool.hit[path_of(i)] = hit; }
     // Material sort: each finished ray's key goes to its queue slot and into
@@ -512,9 +511,10 @@ __device__ __forceinline__ void load_material(const Material* rec, Material& m) 
 
 // shade_surface.slang:59-63: the open guides record this surface.
 __device__ __forceinline__ void record_guides(const PathPool& pool, uint32_t path, float3 w, float3 albedo, float3 n) {
-    float4 a = pool.aov_albedo[path], b = pool.aov_normal[path];
-    pool.aov_albedo[path] = make_float4(a.x + w.x * albedo.x, a.y + w.y * albedo.y, a.z + w.z * albedo.z, a.w);
-    pool.aov_normal[path] = make_float4(b.x + w.x * n.x, b.y + w.y * n.y, b.z + w.z * n.z, b.w);
+    const Float4Pair g = load_pair(&pool.albedo(path));
+    const float4 a = g.a, b = g.b;
+    store_pair(&pool.albedo(path), make_float4(a.x + w.x * albedo.x, a.y + w.y * albedo.y, a.z + w.z * albedo.z, a.w),
+               make_float4(b.x + w.x * n.x, b.y + w.y * n.y, b.z + w.z * n.z, b.w));
 }
 
 __device__ __forceinline__ float luminance(float3 c) { return 0.2722287f * c.x + 0.6740818f * c.y + 0.0536895f * c.z; }
@@ -558,16 +558,15 @@ __global__ void __launch_bounds__(BLOCK, LAYERS ? CN_SHADE_LAYERED_MIN_BLOCKS : 
         uint32_t i = base + lane_id();
         bool push_ray = false, push_shadow = false;
         uint32_t path = 0;
-        ShadowRay sr;
         if (i < count && lane_id() < quota) {
             path = pool.order ? pool.order[i] : (bounce == 0 ? i : queue[i]);
             uint4 h = pool.hit[path];
-            float4 d4 = pool.dir[path];
+            const Float4Pair ray = load_pair(&pool.org(path));
+            const float4 o4 = ray.a, d4 = ray.b;
             float3 dir = xyz(d4);
-            float4 t4 = pool.thr[path];
+            float4 t4 = pool.thr(path);
             float3 thr = xyz(t4);
-            float4 rad = pool.rad[path];
-            if (GUIDE) close_record(pool, path, rad);
+            if (GUIDE) close_record(pool, path, pool.rad(path));
             if (h.x == LIGHT_NONE) {
                 // shade_miss.slang:29-75
                 float weight = 1.0f;
@@ -580,19 +579,21 @@ __global__ void __launch_bounds__(BLOCK, LAYERS ? CN_SHADE_LAYERED_MIN_BLOCKS : 
                     // shade_miss.slang:52-66: depth +inf on a camera ray; the
                     // open guides record the environment as white albedo.
                     const bool camera_ray = t4.w == 0.0f;
-                    if (camera_ray) pool.aov_depth[path] += __int_as_float(0x7f800000);
-                    float3 guide = camera_ray ? f3(1.0f) : xyz(pool.aov_guide[path]);
-                    float4 a = pool.aov_albedo[path];
-                    pool.aov_albedo[path] = make_float4(a.x + guide.x, a.y + guide.y, a.z + guide.z, a.w);
+                    const float4 g4 = pool.aov_guide[path];
+                    if (camera_ray) pool.aov_guide[path].w = g4.w + __int_as_float(0x7f800000);
+                    float3 guide = camera_ray ? f3(1.0f) : xyz(g4);
+                    float4 a = pool.albedo(path);
+                    pool.albedo(path) = make_float4(a.x + guide.x, a.y + guide.y, a.z + guide.z, a.w);
                 }
                 float3 c = thr * env_radiance(scene, dir) * weight;
-                pool.rad[path] = make_float4(rad.x + c.x, rad.y + c.y, rad.z + c.z, rad.w + 1.0f);
+                const float4 rad = pool.rad(path);
+                pool.rad(path) = make_float4(rad.x + c.x, rad.y + c.y, rad.z + c.z, rad.w + 1.0f);
             } else {
                 const uint32_t inst = h.x, prim = h.y;
                 const float b1 = __uint_as_float(h.z), b2 = __uint_as_float(h.w);
                 uint2 ps = pool.ps[path];
                 const uint32_t pixel = ps.x, sample = ps.y;
-                float3 origin = xyz(pool.org[path]);
+                float3 origin = xyz(o4);
                 // The instance record is read field by field where used (all
                 // lanes of a sorted warp mostly share it, so the reads hit L1):
                 // a register copy of it made the kernel spill more.
@@ -615,7 +616,7 @@ __global__ void __launch_bounds__(BLOCK, LAYERS ? CN_SHADE_LAYERED_MIN_BLOCKS : 
                 Spawn sp = sp0;
                 if (normal_map)
                     sp.shading = mapped_shading_normal(scene, inst, prim, uv, mat.normal_texture, sp.shading, sp.normal);
-                uint32_t medium = bounce == 0 ? MEDIUM_NONE : (pool.state[path] & 0xffffffu);
+                uint32_t medium = bounce == 0 ? MEDIUM_NONE : (__float_as_uint(o4.w) & 0xffffffu);
                 if (medium != MEDIUM_NONE) {
                     const Material& in = scene.materials[medium];
                     float depth = __ldg(&in.transmission_depth);
@@ -655,15 +656,20 @@ __global__ void __launch_bounds__(BLOCK, LAYERS ? CN_SHADE_LAYERED_MIN_BLOCKS : 
                 }
                 // Guides (shade_surface.slang:322-340): camera rays are fully
                 // open; the first hit records camera-plane depth.
-                float3 guide = f3(0.0f), aov_alb = f3(0.0f);
+                // The open guides themselves are read where they are spent: held from
+                // here they would spill.
+                float3 aov_alb = f3(0.0f);
                 if (AOV) {
-                    guide = bounce == 0 ? f3(1.0f) : xyz(pool.aov_guide[path]);
-                    if (bounce == 0) pool.aov_depth[path] += length(origin - sp.position) * d4.w;
+                    if (bounce == 0) pool.aov_guide[path].w += length(origin - sp.position) * d4.w;
                     aov_alb = saturate3(cl.aov_albedo);
                 }
                 if (bounce + 1 >= max_bounces) {
-                    if (AOV && any_pos(guide)) record_guides(pool, path, guide, aov_alb, sp.shading);
-                    pool.rad[path] = make_float4(rad.x + contribution.x, rad.y + contribution.y, rad.z + contribution.z,
+                    if (AOV) {
+                        const float3 guide = xyz(pool.aov_guide[path]);
+                        if (any_pos(guide)) record_guides(pool, path, guide, aov_alb, sp.shading);
+                    }
+                    const float4 rad = pool.rad(path);
+                    pool.rad(path) = make_float4(rad.x + contribution.x, rad.y + contribution.y, rad.z + contribution.z,
                                                  rad.w + 1.0f);
                 } else {
                     // Next-event estimation (shade_surface.slang:363-446): one candidate,
@@ -716,16 +722,16 @@ __global__ void __launch_bounds__(BLOCK, LAYERS ? CN_SHADE_LAYERED_MIN_BLOCKS : 
                             float w = mis ? power_heuristic(nee, p_scatter) : 1.0f;
                             float3 unshadowed = thr * crad * ep.f * fabsf(wl.z) * (w / nee);
                             if (any_pos(unshadowed)) {
+                                // Stored at once, in the path's own slot: a compacted slot is only
+                                // known once the warp has converged, and until then the record
+                                // would take 16 registers.
                                 float3 sorg = through ? sp.below : sp.position;
                                 push_shadow = true;
-                                sr.org[0] = sorg.x; sr.org[1] = sorg.y; sr.org[2] = sorg.z;
-                                sr.tmax = ctmax;
-                                sr.dir[0] = cdir.x; sr.dir[1] = cdir.y; sr.dir[2] = cdir.z;
-                                sr.path = path;
-                                sr.contrib[0] = unshadowed.x; sr.contrib[1] = unshadowed.y; sr.contrib[2] = unshadowed.z;
-                                sr.light = clight;
-                                sr.primitive = cprim;
-                                sr.leaf = cleaf;
+                                float4* dst = reinterpret_cast<float4*>(pool.shadows + path);
+                                dst[0] = f4(sorg, ctmax);
+                                dst[1] = f4(cdir, 0.0f);
+                                dst[2] = f4(unshadowed, __uint_as_float(clight));
+                                dst[3] = make_float4(__uint_as_float(cprim), __uint_as_float(cleaf), 0.0f, 0.0f);
                             }
                         }
                     }
@@ -766,9 +772,13 @@ __global__ void __launch_bounds__(BLOCK, LAYERS ? CN_SHADE_LAYERED_MIN_BLOCKS : 
                         if (sample_1d(pixel, sample, bounce_dim(bounce, RR)) >= survival) terminal = true;
                         else scattered = scattered / survival;
                     }
+                    float4 g4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    if (AOV) g4 = pool.aov_guide[path];
+                    const float3 guide = xyz(g4);
                     if (terminal) {
                         if (AOV && any_pos(guide)) record_guides(pool, path, guide, aov_alb, sp.shading);
-                        pool.rad[path] = make_float4(rad.x + contribution.x, rad.y + contribution.y,
+                        const float4 rad = pool.rad(path);
+                        pool.rad(path) = make_float4(rad.x + contribution.x, rad.y + contribution.y,
                                                      rad.z + contribution.z, rad.w + 1.0f);
                     } else {
                         if (AOV) {
@@ -776,14 +786,15 @@ __global__ void __launch_bounds__(BLOCK, LAYERS ? CN_SHADE_LAYERED_MIN_BLOCKS : 
                             // open guides between this surface and the scattered ray.
                             float rec = aov_record_fraction(cl, sc.lobe);
                             if (rec > 0.0f && any_pos(guide)) record_guides(pool, path, guide * rec, aov_alb, sp.shading);
-                            pool.aov_guide[path] = f4(guide * (1.0f - rec) * aov_pass_tint(cl, sc.lobe), 0.0f);
+                            pool.aov_guide[path] = f4(guide * (1.0f - rec) * aov_pass_tint(cl, sc.lobe), g4.w);
                         }
                         if (sc.lobe == LOBE_TRANSMISSION && mat.thin_walled == 0)
                             medium = medium == inst ? MEDIUM_NONE : inst;
-                        pool.org[path] = f4(sc.wi.z < 0.0f ? sp.below : sp.position, 0.0f);
-                        pool.dir[path] = f4(wiw, 0.0f);
-                        pool.thr[path] = f4(scattered, sc.pdf);
-                        pool.state[path] = (sc.lobe << 24) | (medium & 0xffffffu);
+                        store_pair(&pool.org(path),
+                                   f4(sc.wi.z < 0.0f ? sp.below : sp.position,
+                                      __uint_as_float((sc.lobe << 24) | (medium & 0xffffffu))),
+                                   f4(wiw, 0.0f));
+                        pool.thr(path) = f4(scattered, sc.pdf);
                         push_ray = true;
                         if (GUIDE && g_alpha > 0.0f && pool.sink->records &&
                             hash_uniform(pixel, sample, bounce, 0x6a09u) < pool.sink->rate) {
@@ -798,30 +809,24 @@ __global__ void __launch_bounds__(BLOCK, LAYERS ? CN_SHADE_LAYERED_MIN_BLOCKS : 
                                 pool.guide_rec[path] = idx;
                             }
                         }
-                        if (any_pos(contribution))
-                            pool.rad[path] =
+                        if (any_pos(contribution)) {
+                            const float4 rad = pool.rad(path);
+                            pool.rad(path) =
                                 make_float4(rad.x + contribution.x, rad.y + contribution.y, rad.z + contribution.z, rad.w);
+                        }
                     }
                 }
             }
         }
-        uint32_t slot = warp_push(pool.counters + CTR_RAYS + bounce + 1, push_ray);
+        const uint2 slot = warp_push2(pool.counters + CTR_RAYS + bounce + 1, push_ray,
+                                      pool.counters + CTR_SHADOWS + bounce, push_shadow);
         if (push_ray) {
-            if (slot < pool.capacity) next_queue[slot] = path;
+            if (slot.x < pool.capacity) next_queue[slot.x] = path;
             else flag_overflow(pool.counters);
         }
-        uint32_t sslot = warp_push(pool.counters + CTR_SHADOWS + bounce, push_shadow);
         if (push_shadow) {
-            if (sslot < pool.capacity) {
-                float4* dst = reinterpret_cast<float4*>(pool.shadows + sslot);
-                const float4* src = reinterpret_cast<const float4*>(&sr);
-                dst[0] = src[0];
-                dst[1] = src[1];
-                dst[2] = src[2];
-                dst[3] = src[3];
-            } else {
-                flag_overflow(pool.counters);
-            }
+            if (slot.y < pool.capacity) pool.shadow_queue[slot.y] = path;
+            else flag_overflow(pool.counters);
         }
         if (first + ws.rest >= count) break;
         base = first + ws.rest + warp_fetch(fetch);
@@ -849,9 +854,9 @@ __global__ void __launch_bounds__(B, CN_TRAV_MIN_BLOCKS * BLOCK / B)
         if (!drained) {
             uint32_t i = refill(fetch, count, live, drained, rest);
             if (i != ~0u) {
-                const float4* rec = reinterpret_cast<const float4*>(pool.shadows + i);
+                path = pool.shadow_queue[i];
+                const float4* rec = reinterpret_cast<const float4*>(pool.shadows + path);
                 float4 q0 = rec[0], q1 = rec[1], q2 = rec[2], q3 = rec[3];
-                path = __float_as_uint(q1.w);
                 contrib = xyz(q2);
                 ray = make_ray(xyz(q0), xyz(q1));
                 shadow_begin(scene, ray, q0.w, __float_as_uint(q2.w), __float_as_uint(q3.x), __float_as_uint(q3.y), q);
@@ -872,8 +877,8 @@ __global__ void __launch_bounds__(B, CN_TRAV_MIN_BLOCKS * BLOCK / B)
                 } else if (st == WALK_DONE) {
                     float atten = shadow_result(q);
                     if (atten >= 0.0f) {
-                        float4 r = pool.rad[path];
-                        pool.rad[path] = make_float4(r.x + contrib.x * atten, r.y + contrib.y * atten,
+                        float4 r = pool.rad(path);
+                        pool.rad(path) = make_float4(r.x + contrib.x * atten, r.y + contrib.y * atten,
                                                      r.z + contrib.z * atten, r.w);
                     }
                     live = false;
@@ -901,7 +906,7 @@ struct ShadowSource {
         return refill(fetch, count, live, drained, rest);
     }
     __device__ __forceinline__ bool begin(uint32_t i, Ray& ray, AnyQuery& a) const {
-        const float4* rec = reinterpret_cast<const float4*>(pool.shadows + i);
+        const float4* rec = reinterpret_cast<const float4*>(pool.shadows + pool.shadow_queue[i]);
         const float4 q0 = rec[0], q1 = rec[1], q2 = rec[2], q3 = rec[3];
         ray = make_ray(xyz(q0), xyz(q1));
         const uint32_t light = __float_as_uint(q2.w), leaf = __float_as_uint(q3.y);
@@ -920,10 +925,9 @@ struct ShadowSource {
         return true;
     }
     __device__ __forceinline__ void add(uint32_t i, float atten) const {
-        const float4* rec = reinterpret_cast<const float4*>(pool.shadows + i);
-        const uint32_t path = __float_as_uint(rec[1].w);
-        const float4 c = rec[2], r = pool.rad[path];
-        pool.rad[path] = make_float4(r.x + c.x * atten, r.y + c.y * atten, r.z + c.z * atten, r.w);
+        const uint32_t path = pool.shadow_queue[i];
+        const float4 c = reinterpret_cast<const float4*>(pool.shadows + path)[2], r = pool.rad(path);
+        pool.rad(path) = make_float4(r.x + c.x * atten, r.y + c.y * atten, r.z + c.z * atten, r.w);
     }
     __device__ __forceinline__ void emit(uint32_t i, bool visible) const {
         if (visible) add(i, 1.0f);
@@ -975,12 +979,13 @@ __global__ void k_accumulate(PathPool pool, FilmTargets film, uint32_t pixel_bas
         }
         for (uint32_t s = 0; s < samples; ++s) {
             const size_t q = size_t(s) * count + p;
-            float4 v = pool.rad[q];
+            float4 v = pool.rad(q);
             if (!finite4(v)) v = zero;
             acc = (reset && s == 0) ? v : add4(acc, v);
             if (AOV) {
-                float4 a = pool.aov_albedo[q], n = pool.aov_normal[q];
-                float d = pool.aov_depth[q];
+                const Float4Pair g = load_pair(&pool.albedo(q));
+                float4 a = g.a, n = g.b;
+                float d = pool.aov_guide[q].w;
                 if (!finite4(a)) a = zero;
                 if (!finite4(n)) n = zero;
                 if (isnan(d)) d = 0.0f;
@@ -1013,7 +1018,7 @@ __global__ void k_accumulate_segments(PathPool pool, const WaveSegment* __restri
         const uint32_t p = x - g.pixel_start, px = g.pixel_base + p;
         float4 acc = g.reset ? zero : g.film[px];
         for (uint32_t s = 0; s < g.samples; ++s) {
-            float4 v = pool.rad[g.start + s * g.pixel_count + p];
+            float4 v = pool.rad(g.start + s * g.pixel_count + p);
             if (!finite4(v)) v = zero;
             acc = (g.reset && s == 0) ? v : add4(acc, v);
         }
@@ -1068,10 +1073,10 @@ __global__ void k_resolve1(const float* __restrict__ sum, float* __restrict__ av
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) avg[p] = sum[p] / samples;
 }
 
-__global__ void k_copy_rad(const float4* __restrict__ rad, float4* __restrict__ out, uint32_t base, uint32_t count,
+__global__ void k_copy_rad(PathPool pool, float4* __restrict__ out, uint32_t base, uint32_t count,
                            uint32_t tile_width) {
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < count; p += gridDim.x * blockDim.x)
-        out[base + wave_pixel(p, tile_width)] = rad[p];
+        out[base + wave_pixel(p, tile_width)] = pool.rad(p);
 }
 
 // ---- material sort -----------------------------------------------------------------
@@ -1306,7 +1311,7 @@ void launch_intersect(const DeviceScene& scene, const PathPool& pool, uint32_t b
 
 void launch_shade(const DeviceScene& scene, const PathPool& pool, uint32_t bounce, const WaveParams& wp, uint32_t n0,
                   const LaunchShape& ls, cudaStream_t stream) {
-    const bool aov = pool.aov_albedo != nullptr, guided = pool.guide_out != nullptr;
+    const bool aov = pool.aov != nullptr, guided = pool.guide_out != nullptr;
     auto shade = [&](bool layers, uint32_t part) {
         auto args = [&](auto kernel) {
             kernel<<<layers ? ls.grid_shade : ls.grid_shade_free, BLOCK, 0, stream>>>(
@@ -1361,7 +1366,7 @@ void launch_accumulate(const PathPool& pool, const FilmTargets& film, uint32_t p
                        uint32_t tile_width, uint32_t samples, bool reset, cudaStream_t stream) {
     int grid = int((pixel_count + 255) / 256);
     if (grid > 148 * 16) grid = 148 * 16;
-    if (pool.aov_albedo && film.albedo)
+    if (pool.aov && film.albedo)
         k_accumulate<true><<<grid, 256, 0, stream>>>(pool, film, pixel_base, pixel_count, tile_width, samples,
                                                      reset ? 1u : 0u);
     else
@@ -1402,7 +1407,7 @@ void launch_copy_rad(const PathPool& pool, float4* out, uint32_t pixel_base, uin
                      cudaStream_t stream) {
     int grid = int((pixel_count + 255) / 256);
     if (grid > 148 * 16) grid = 148 * 16;
-    k_copy_rad<<<grid, 256, 0, stream>>>(pool.rad, out, pixel_base, pixel_count, tile_width);
+    k_copy_rad<<<grid, 256, 0, stream>>>(pool, out, pixel_base, pixel_count, tile_width);
 }
 
 }  // namespace cn
