@@ -537,14 +537,14 @@ class Film:
 
     def averages(self, out: np.ndarray | None = None) -> np.ndarray:
         if out is None:
-            out = np.zeros((self.height, self.width, 4), np.float32)
+            out = np.empty((self.height, self.width, 4), np.float32)
         _check(library().cenote_film_averages(self._h, _ptr(out), None, None, None))
         return out
 
     def all_averages(self) -> dict:
         """Film::averages (film.rs:183-191): beauty, albedo, normal (H, W, 4) and depth (H, W)."""
-        out = {k: np.zeros((self.height, self.width, 4), np.float32) for k in ("beauty", "albedo", "normal")}
-        out["depth"] = np.zeros((self.height, self.width), np.float32)
+        out = {k: np.empty((self.height, self.width, 4), np.float32) for k in ("beauty", "albedo", "normal")}
+        out["depth"] = np.empty((self.height, self.width), np.float32)
         _check(library().cenote_film_averages(self._h, _ptr(out["beauty"]), _ptr(out["albedo"]), _ptr(out["normal"]),
                                               _ptr(out["depth"])))
         return out
@@ -555,7 +555,7 @@ class Film:
 
     def tonemap(self, exposure_stops: float = 0.0) -> np.ndarray:
         """The display frame (tonemap.slang): uint8 (H, W, 4), sRGB-encoded."""
-        out = np.zeros((self.height, self.width), np.uint32)
+        out = np.empty((self.height, self.width), np.uint32)
         _check(library().cenote_film_tonemap(self._h, exposure_stops, _ptr(out)))
         return out.view(np.uint8).reshape(self.height, self.width, 4)
 
@@ -572,7 +572,7 @@ class Film:
         _check(library().cenote_film_restore(self._h, _ptr(s), samples))
 
     def sums(self) -> np.ndarray:
-        out = np.zeros((self.height, self.width, 4), np.float32)
+        out = np.empty((self.height, self.width, 4), np.float32)
         _check(library().cenote_film_sums(self._h, _ptr(out)))
         return out
 
@@ -638,7 +638,7 @@ class Renderer:
         return {name: getattr(t, name) for name, _ in TuningC._fields_}
 
     def render(self, scene: Scene, width: int, height: int, sample: int = 0) -> np.ndarray:
-        out = np.zeros((height, width, 4), np.float32)
+        out = np.empty((height, width, 4), np.float32)
         _check(library().cenote_render_once(self._h, scene.handle, width, height, sample, _ptr(out)))
         return out
 

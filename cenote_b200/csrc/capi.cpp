@@ -270,6 +270,7 @@ int32_t cenote_context_create(const cenote_options* options, cenote_context** ou
     ctx->shape = launch_shape(dev);
     ctx->l2_persist_max = size_t(prop.persistingL2CacheMaxSize);
     ctx->l2_window_max = size_t(prop.accessPolicyMaxWindowSize);
+    CN_CUDA(cudaMallocHost(reinterpret_cast<void**>(&ctx->tally_host), 4096));
     CN_CUDA(ctx->tables.alloc(sizeof(kTables)));
     CN_CUDA(cudaMemcpy(ctx->tables.ptr, kTables, sizeof(kTables), cudaMemcpyHostToDevice));
     *out = ctx.release();
@@ -1087,10 +1088,11 @@ int32_t run_waves(cenote_renderer* r, cenote_scene* sc, uint32_t width, uint32_t
     CN_CUDA(enqueue_waves(r, sc, width, height, sample0, count, r->max_bounces, plan, film ? &targets : nullptr,
                           film && film->samples == 0, oneshot, nullptr, ctx->stream, timing, counting, &wc));
     CN_CUDA(cudaEventRecord(ctx->t1, ctx->stream));
+    unsigned long long t[6];
+    CN_CUDA(cudaMemcpyAsync(ctx->tally_host, r->tally.ptr, sizeof t, cudaMemcpyDeviceToHost, ctx->stream));
     int32_t rc = wait_stream(ctx->stream, ctx->sync_ev, 600000.0);
     if (rc != CENOTE_OK) return rc;
-    unsigned long long t[6];
-    CN_CUDA(cudaMemcpy(t, r->tally.ptr, sizeof t, cudaMemcpyDeviceToHost));
+    std::memcpy(t, ctx->tally_host, sizeof t);
     float ms = 0.0f;
     cudaEventElapsedTime(&ms, ctx->t0, ctx->t1);
     cenote_stats st{};
@@ -1267,13 +1269,11 @@ int32_t cenote_render_once(cenote_renderer* r, cenote_scene* scene, uint32_t wid
     CN_CHECK(uint64_t(width) * height < (1ull << 31), CENOTE_E_INVALID_ARGUMENT, "target too large");
     std::lock_guard<std::mutex> lock(r->ctx->mu);
     CN_CUDA(cudaSetDevice(r->ctx->device));
-    DeviceBuffer out;
-    size_t bytes = size_t(width) * height * 16;
-    CN_CUDA(out.alloc(bytes));
-    int32_t rc = run_waves(r, scene, width, height, sample, 1, nullptr, out.as<float4>());
+    const size_t bytes = size_t(width) * height * 16;
+    if (r->oneshot.bytes < bytes) CN_CUDA(r->oneshot.alloc(bytes));
+    int32_t rc = run_waves(r, scene, width, height, sample, 1, nullptr, r->oneshot.as<float4>());
     if (rc != CENOTE_OK) return rc;
-    CN_CUDA(cudaMemcpy(rgba_out, out.ptr, bytes, cudaMemcpyDeviceToHost));
-    return CENOTE_OK;
+    return copy_out(r->ctx, rgba_out, r->oneshot.ptr, bytes);
 }
 
 int32_t cenote_film_averages(cenote_film* film, float* beauty, float* albedo, float* normal, float* depth) {
@@ -1285,7 +1285,7 @@ int32_t cenote_film_averages(cenote_film* film, float* beauty, float* albedo, fl
         launch_resolve(film->sum.as<float4>(), film->avg.as<float4>(), uint32_t(px), float(std::max(1u, film->samples)),
                        film->ctx->stream);
         CN_CUDA(cudaGetLastError());
-        CN_CUDA(cudaMemcpyAsync(beauty, film->avg.ptr, px * 16, cudaMemcpyDeviceToHost, film->ctx->stream));
+        if (int32_t rc = copy_out(film->ctx, beauty, film->avg.ptr, px * 16)) return rc;
     }
     const float n = float(std::max(1u, film->samples));
     float4* avg = film->avg.as<float4>();
@@ -1294,12 +1294,12 @@ int32_t cenote_film_averages(cenote_film* film, float* beauty, float* albedo, fl
         if (!dst) continue;
         launch_resolve(src, avg, uint32_t(px), n, film->ctx->stream);
         CN_CUDA(cudaGetLastError());
-        CN_CUDA(cudaMemcpyAsync(dst, avg, px * 16, cudaMemcpyDeviceToHost, film->ctx->stream));
+        if (int32_t rc = copy_out(film->ctx, dst, avg, px * 16)) return rc;
     }
     if (depth) {
         launch_resolve1(film->depth.as<float>(), film->avg.as<float>(), uint32_t(px), n, film->ctx->stream);
         CN_CUDA(cudaGetLastError());
-        CN_CUDA(cudaMemcpyAsync(depth, film->avg.ptr, px * 4, cudaMemcpyDeviceToHost, film->ctx->stream));
+        if (int32_t rc = copy_out(film->ctx, depth, film->avg.ptr, px * 4)) return rc;
     }
     return wait_stream(film->ctx->stream, film->ctx->sync_ev, 600000.0);
 }
@@ -1326,17 +1326,14 @@ int32_t cenote_film_tonemap(cenote_film* film, float exposure_stops, uint32_t* r
     CN_CUDA(out.alloc(px * 4));
     int32_t rc = cenote_film_tonemap_device(film, exposure_stops, out.ptr);
     if (rc != CENOTE_OK) return rc;
-    CN_CUDA(cudaMemcpyAsync(rgba8, out.ptr, px * 4, cudaMemcpyDeviceToHost, film->ctx->stream));
-    return wait_stream(film->ctx->stream, film->ctx->sync_ev, 600000.0);
+    return copy_out(film->ctx, rgba8, out.ptr, px * 4);
 }
 
 int32_t cenote_film_sums(cenote_film* film, float* beauty_sum) {
     CN_CHECK(film && beauty_sum, CENOTE_E_INVALID_ARGUMENT, "null argument");
     std::lock_guard<std::mutex> lock(film->ctx->mu);
     CN_CUDA(cudaSetDevice(film->ctx->device));
-    CN_CUDA(cudaMemcpyAsync(beauty_sum, film->sum.ptr, size_t(film->width) * film->height * 16, cudaMemcpyDeviceToHost,
-                            film->ctx->stream));
-    return wait_stream(film->ctx->stream, film->ctx->sync_ev, 600000.0);
+    return copy_out(film->ctx, beauty_sum, film->sum.ptr, size_t(film->width) * film->height * 16);
 }
 
 int32_t cenote_film_restore(cenote_film* film, const float* beauty_sum, uint32_t samples) {

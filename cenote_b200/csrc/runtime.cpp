@@ -50,8 +50,16 @@ int32_t wait_event(cudaEvent_t ev, double timeout_ms) {
         if (e != cudaErrorNotReady) return fail(CENOTE_E_DEVICE, std::string("device error: ") + cudaGetErrorString(e));
         double ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
         if (ms > timeout_ms) return fail(CENOTE_E_TIMEOUT, "device work did not finish within the wait bound");
-        std::this_thread::sleep_for(std::chrono::microseconds(ms < 5.0 ? 20 : 200));
+        // A sleep of 20 us ends about 80 us later (the timer's slack): calls of
+        // a millisecond or two poll instead, long ones give the core back.
+        if (ms < 2.0) std::this_thread::yield();
+        else std::this_thread::sleep_for(std::chrono::microseconds(ms < 20.0 ? 20 : 200));
     }
+}
+
+int32_t copy_out(cenote_context* ctx, void* host, const void* device, size_t bytes) {
+    CN_CUDA(cudaMemcpyAsync(host, device, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+    return wait_stream(ctx->stream, ctx->sync_ev, 600000.0);
 }
 
 // How a call splits into waves: `range` pixels per wave, `spw` samples each.

@@ -19,6 +19,12 @@
 
 namespace cn {
 
+}  // namespace cn
+
+struct cenote_context;
+
+namespace cn {
+
 // Record `msg` as this thread's last error and return `code`.
 int32_t fail(int32_t code, const std::string& msg);
 // The calling thread's last error message (cenote_last_error).
@@ -41,6 +47,9 @@ const char* last_error();
 // `timeout_ms` passes (CENOTE_E_TIMEOUT).
 int32_t wait_stream(cudaStream_t s, cudaEvent_t ev, double timeout_ms);
 int32_t wait_event(cudaEvent_t ev, double timeout_ms);
+
+// Device memory to the caller's host memory on the context's stream, waited for.
+int32_t copy_out(cenote_context* ctx, void* host, const void* device, size_t bytes);
 
 struct DeviceBuffer {
     void* ptr = nullptr;
@@ -90,6 +99,7 @@ struct cenote_context {
     LaunchShape shape{};
     cn::DeviceBuffer tables;
     std::mutex mu;
+    unsigned long long* tally_host = nullptr;  // pinned: a wave's counters come back with its last event
     // L2 persistence (this context's own set-aside; nothing outlives it).
     size_t l2_persist_max = 0, l2_window_max = 0, l2_set_aside = 0;
     uint32_t bvh_builder = CENOTE_BVH_AUTO;  // for scenes created from now on
@@ -165,6 +175,7 @@ struct cenote_renderer {
     uint32_t sort_by_location = 0;    // 1: the material sort keys layer-free hits by location
     float tuned_ms_per_sample = 0.0f;
     DeviceBuffer sort_order, sort_keys, sort_bins;
+    DeviceBuffer oneshot;  // a one-shot render's image
     DeviceBuffer aov, aov_guide;
     size_t pool_cap = 0, aov_cap = 0;
     // The learned guide (cenote_renderer_set_guide): per-path mixture outputs
@@ -337,6 +348,7 @@ inline void free_context(cenote_context* ctx) {
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     ctx->tables.release();
     if (ctx->sync_ev) cudaEventDestroy(ctx->sync_ev);
+    if (ctx->tally_host) cudaFreeHost(ctx->tally_host);
     if (ctx->t0) cudaEventDestroy(ctx->t0);
     if (ctx->t1) cudaEventDestroy(ctx->t1);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
