@@ -72,9 +72,29 @@ WavePlan plan_waves(const cenote_renderer* r, uint64_t pixels, uint32_t count, b
         p.spw = r->samples_per_wave;
     } else {
         // Enough paths per wave to keep 148 SMs busy through the tail bounces
-        // and amortise each bounce's launches (16 M paths, ~4 GB of path
-        // state; on the chart 4 M-path waves left intersect 20 % slower).
-        uint64_t want = (uint64_t(1) << 24) / pixels;
+        // and amortise each bounce's launches: every wave ends in bounces of
+        // few paths. Up to 64 M paths (14.5 GB of path state) while the pool
+        // holds them or they take at most an eighth of the free memory, and
+        // 16 M (3.6 GB) in any case. The terrain's 64-spp frame takes 238, 228
+        // and 222 ms in waves of 16, 33 and 66 M paths, the chart's 56.6, 54.9
+        // and 54.1 in waves of 17, 33 and 59 M. A guide that trains once per
+        // wave keeps the 16 M of its schedule.
+        uint64_t paths = uint64_t(1) << 24;
+        if (!oneshot && !r->guide && pixels * count > paths) {
+            size_t free_bytes = 0, total = 0;
+            for (uint64_t big : {uint64_t(1) << 26, uint64_t(1) << 25}) {
+                const uint64_t need = std::min<uint64_t>(big, pixels * count);
+                if (need > r->pool_cap && !free_bytes && cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) {
+                    cudaGetLastError();
+                    break;
+                }
+                if (need <= r->pool_cap || need * cenote_renderer::PATH_BYTES <= free_bytes / 8) {
+                    paths = big;
+                    break;
+                }
+            }
+        }
+        uint64_t want = paths / pixels;
         p.spw = uint32_t(std::max<uint64_t>(1, std::min<uint64_t>(want, 64)));
     }
     if (oneshot) p.spw = 1;

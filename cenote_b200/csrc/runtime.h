@@ -185,6 +185,8 @@ struct cenote_renderer {
     uint32_t guide_steps = 0;
     DeviceBuffer g_out, g_rec, g_records, g_count, g_sink;
     size_t g_cap = 0;
+    // Device bytes a path of the pool takes with the denoiser guides' lanes.
+    static constexpr uint64_t PATH_BYTES = 32 * 2 + 16 + 8 + 8 + sizeof(ShadowRay) + 4 + 8 + 48;
     static constexpr uint32_t GUIDE_RECORDS = 1u << 20;
     static constexpr uint32_t GUIDE_BATCH = 65536;
     // The shadow walks' own stream and the events that fork it off the main

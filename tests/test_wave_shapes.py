@@ -33,3 +33,25 @@ def test_film_is_the_same_in_any_wave(ctx, name, w, h, spp, bounces):
         assert n == rays, kw
         for k in base:
             assert np.array_equal(got[k], base[k], equal_nan=True), (kw, k)
+
+
+def test_one_large_wave_is_the_small_waves(ctx):
+    """More than 2^24 paths go in one wave where memory is plentiful; a guide
+    that trains per wave keeps its 2^24; the films are the same bits."""
+    from cenote_b200 import Guide
+
+    scene = Scene(ctx, scenes.cornell())
+    r, f = Renderer(ctx, 3), Film(ctx, 1024, 1024)
+    r.accumulate(scene, f, 17)
+    assert r.stats()["samples_per_wave"] == 17
+    base = f.all_averages()
+    r.set_samples_per_wave(16)
+    f.reset()
+    r.accumulate(scene, f, 17)
+    for k, v in f.all_averages().items():
+        assert np.array_equal(v, base[k], equal_nan=True), k
+    guided = Renderer(ctx, 2)
+    guided.set_guide(Guide(ctx, 1), 0.5, 0)
+    f.reset()
+    guided.accumulate(scene, f, 17)
+    assert guided.stats()["samples_per_wave"] == 16
