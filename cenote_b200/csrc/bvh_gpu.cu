@@ -934,7 +934,8 @@ __global__ void k_light_leaves(const float4* __restrict__ tris, uint32_t n, cons
 }
 
 // One thread per triangle of the concatenated meshes: its instance by binary
-// search, its corners gathered through the instance's indices.
+// search, its corners gathered through the instance's indices. Runs once per
+// scene, bound by the upload before it.
 __global__ void k_attributes(const float* __restrict__ positions, const float* __restrict__ normals,
                              const float* __restrict__ uvs, const uint32_t* __restrict__ indices,
                              const uint32_t* __restrict__ first_tri, const uint64_t* __restrict__ first_vertex,

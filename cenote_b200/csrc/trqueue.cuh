@@ -10,10 +10,10 @@
 // per-warp FIFO in shared memory and keeps walking; once the FIFO holds a
 // warp's worth of triangles (or no lane has nodes left), a round hands one
 // (ray, triangle) pair to every lane: a warp scan of the entries' bit counts
-// maps lane j to its entry and bit, the owner's ray comes over shuffles, and
-// each owner's candidates reduce to the lexicographic minimum of (t,
-// instance, primitive) through shared-memory atomic minima (any-hit queries:
-// an OR of occluders). A lane whose walk has ended waits for its queued
+// maps lane j to its entry and bit, the owner's ray comes over shuffles and
+// shared memory, and each owner's candidates reduce to the lexicographic
+// minimum of (t, instance, primitive) through a shared-memory atomic minimum
+// (any-hit queries: an OR of occluders). A lane whose walk has ended waits for its queued
 // triangles before it takes a new ray.
 //
 // Results are bitwise those of the per-lane walk: the watertight test of a

@@ -26,6 +26,7 @@
 #include "textures.cuh"
 #include "traverse.cuh"
 #include "trqueue.cuh"
+#include "trwide.cuh"
 
 namespace cn {
 
@@ -47,8 +48,9 @@ constexpr int BLOCK = 128;
 #ifndef CN_SHADE_LAYERED_MIN_BLOCKS
 #define CN_SHADE_LAYERED_MIN_BLOCKS 4
 #endif
-// The same for the traversal kernels (8 → 64 registers), and for the
-// closest-hit walks alone (which spill a little at 64 registers).
+// The same for the traversal kernels (8 → 64 registers, the queued walks
+// without spills; 9 and 10 were level and 7 % slower on the terrain), and for
+// the closest-hit walks alone.
 #ifndef CN_TRAV_MIN_BLOCKS
 #define CN_TRAV_MIN_BLOCKS 8
 #endif
@@ -259,6 +261,15 @@ __device__ __forceinline__ uint32_t lanemask_lt() { return (1u << lane_id()) - 1
 #define CN_QUOTA_SHADE 1
 #endif
 
+// Up to this many rays a warp, the queued walks give each ray eight lanes
+// (trwide.cuh). Device ms of the one-sample 640x360 chart frame and the
+// two-sample 853x479 terrain frame without it and at 1, 4, 8 and 16: 0.902,
+// 0.841, 0.807, 0.815, 0.823 and 3.47, 3.31, 3.29, 3.28, 3.28; the closed box
+// (its bounces rarely short) slows from 8 on.
+#ifndef CN_WIDE_RAYS
+#define CN_WIDE_RAYS 4
+#endif
+
 // Hand the warp's idle lanes their next work items: returns this lane's item
 // index (or ~0u) and sets `drained` (warp-uniform) once the queue is used up.
 // `rest` is 0 before the warp's first batch (warp_share) and the first item
@@ -444,9 +455,13 @@ __global__ void __launch_bounds__(B, CN_ISECT_MIN_BLOCKS * BLOCK / B)
     IsectSource src{pool, &scene, pool.queue[bounce & 1u], pool.counters + CTR_FETCH_ISECT + bounce,
                     bounce_paths(pool, bounce, n0), bounce};
     bool overflow = false;
-    queued_closest<COUNT, IsectSource, S>(scene, tqs[threadIdx.x >> 5], src,
-                                          bounce == 0 ? RAY_MASK_CAMERA : RAY_MASK_ALL, overflow,
-                          &visits, &tests);
+    const uint32_t mask = bounce == 0 ? RAY_MASK_CAMERA : RAY_MASK_ALL;
+    const WarpShare ws = warp_share(src.count, 1u);
+    if (ws.quota <= CN_WIDE_RAYS)
+        wide_closest<COUNT>(scene, tqs[threadIdx.x >> 5], src, ws.first, min(ws.first + ws.quota, src.count), mask,
+                            overflow, &visits, &tests);
+    else
+        queued_closest<COUNT, IsectSource, S>(scene, tqs[threadIdx.x >> 5], src, mask, overflow, &visits, &tests);
     if (overflow) flag_overflow(pool.counters);
     if (COUNT) flush_counts(pool.counters, visits, tests);
 }
@@ -950,7 +965,12 @@ __global__ void __launch_bounds__(B, CN_TRAV_MIN_BLOCKS * BLOCK / B)
     ShadowSource src{scene, pool, pool.counters + CTR_FETCH_SHADOW + bounce,
                      min(pool.counters[CTR_SHADOWS + bounce], pool.capacity)};
     bool overflow = false;
-    queued_any<COUNT, ShadowSource, S>(scene, tqs[threadIdx.x >> 5], src, overflow, &visits, &tests);
+    const WarpShare ws = warp_share(src.count, 1u);
+    if (ws.quota <= CN_WIDE_RAYS)
+        wide_any<COUNT>(scene, tqs[threadIdx.x >> 5], src, ws.first, min(ws.first + ws.quota, src.count), overflow,
+                        &visits, &tests);
+    else
+        queued_any<COUNT, ShadowSource, S>(scene, tqs[threadIdx.x >> 5], src, overflow, &visits, &tests);
     if (overflow) flag_overflow(pool.counters);
     if (COUNT) flush_counts(pool.counters, visits, tests);
 }

@@ -62,3 +62,38 @@ def test_edge_rays_hit_as_the_oracle_says(ctx, scale, offset):
             hits, t = dev.probe_intersect(org, d, queued=queued)
             assert np.array_equal(hits, rh)
             assert np.array_equal(t, rt)
+
+
+@pytest.mark.parametrize("name", ["stacked", "chart", "cornell", "axis_light"])
+@pytest.mark.parametrize("w,h,spp", [(1, 1, 1), (5, 1, 1), (67, 71, 1), (67, 71, 3), (137, 138, 1), (160, 120, 4)])
+def test_short_queues_walk_to_the_same_hits(ctx, name, w, h, spp):
+    """A queue of at most a few rays per warp is walked by eight lanes a ray,
+    longer ones by a lane a ray with shared triangle tests, and on request by
+    a lane a ray alone: the films and ray counts are the same, bit for bit,
+    with coincident surfaces, axis-parallel rays and shadow rays to a target
+    or to none. The sizes straddle the lengths where the walk changes."""
+    from cenote_b200 import Film, Renderer
+
+    if name == "stacked":
+        spec = stacked(1.0, (0, 0, 0))
+        spec.objects.append(scenes.Object(scenes.quad([(-1, 3, -1), (1, 3, -1), (1, 3, 1), (-1, 3, 1)]),
+                                          scenes.rows(np.eye(4)), scenes.emitter((5.0, 5.0, 5.0))))
+        spec.camera = scenes.Camera((2.5, 2.0, 3.0), (0.0, 0.0, 0.0))
+    elif name == "axis_light":  # a distant light straight down: every shadow ray is axis-parallel
+        spec = scenes.chart(env_size=(8, 4))
+        spec.delta_lights = [scenes.DeltaLight(1, (0.0, -1.0, 0.0), (3.0, 3.0, 3.0))]
+    else:
+        spec = {"chart": lambda: scenes.chart(env_size=(64, 32)), "cornell": scenes.cornell}[name]()
+    scene = Scene(ctx, spec)
+    films = []
+    for per_lane in (0, 1):
+        r, f = Renderer(ctx, 8), Film(ctx, w, h)
+        r.set_tuning(0, per_lane_triangles=per_lane)
+        r.accumulate(scene, f, spp)
+        st = r.stats()
+        assert st["overflow"] == 0
+        films.append((f.all_averages(), st["extension_rays"], st["shadow_rays"]))
+    (a, *na), (b, *nb) = films
+    assert na == nb
+    for k in a:
+        assert np.array_equal(a[k], b[k], equal_nan=True), k
