@@ -526,21 +526,26 @@ int32_t cenote_scene_create_textured(cenote_context* ctx, const cenote_object* o
     const uint32_t tri_count = uint32_t(tris.size());
     DeviceBuffer* battrs = sc->add(size_t(tri_count) * TRI_ATTRS * 16, &err);
     CN_CUDA(err);
-    DeviceBuffer mesh_stage[6];
+    DeviceBuffer mesh_stage;  // the six streams in one allocation (each one freed here waits for the device)
     {
         const std::pair<const void*, size_t> streams[6] = {
             {positions.data(), positions.size() * 4}, {normals.data(), normals.size() * 4},
             {uvs.data(), uvs.size() * 4},             {indices.data(), indices.size() * 4},
             {first_tri.data(), first_tri.size() * 4}, {first_vertex.data(), first_vertex.size() * 8}};
-        for (int k = 0; k < 6; ++k) {
-            CN_CUDA(mesh_stage[k].alloc(streams[k].second));
+        size_t at[7] = {0};
+        for (int k = 0; k < 6; ++k) at[k + 1] = at[k] + (streams[k].second + 255) / 256 * 256;
+        CN_CUDA(mesh_stage.alloc(at[6]));
+        uint8_t* stage = mesh_stage.as<uint8_t>();
+        for (int k = 0; k < 6; ++k)
             if (streams[k].second)
-                CN_CUDA(cudaMemcpyAsync(mesh_stage[k].ptr, streams[k].first, streams[k].second, cudaMemcpyHostToDevice,
+                CN_CUDA(cudaMemcpyAsync(stage + at[k], streams[k].first, streams[k].second, cudaMemcpyHostToDevice,
                                         ctx->stream));
-        }
-        launch_attributes(mesh_stage[0].as<float>(), mesh_stage[1].as<float>(), mesh_stage[2].as<float>(),
-                          mesh_stage[3].as<uint32_t>(), mesh_stage[4].as<uint32_t>(), mesh_stage[5].as<uint64_t>(),
-                          object_count, tri_count, battrs->as<float4>(), ctx->stream);
+        launch_attributes(reinterpret_cast<const float*>(stage + at[0]), reinterpret_cast<const float*>(stage + at[1]),
+                          reinterpret_cast<const float*>(stage + at[2]),
+                          reinterpret_cast<const uint32_t*>(stage + at[3]),
+                          reinterpret_cast<const uint32_t*>(stage + at[4]),
+                          reinterpret_cast<const uint64_t*>(stage + at[5]), object_count, tri_count,
+                          battrs->as<float4>(), ctx->stream);
         CN_CUDA(cudaGetLastError());
     }
     for (uint32_t i = 0; i < object_count; ++i) geoms[i].attrs = battrs->as<float4>() + size_t(first_tri[i]) * TRI_ATTRS;
