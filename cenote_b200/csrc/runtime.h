@@ -222,7 +222,8 @@ struct cenote_renderer {
 
     // The sort mode of a wave of `paths` camera paths (0: known on the device
     // only). Unless a mode was chosen, waves whose bounces shade no faster in
-    // material order skip it; films are the same bits either way where the
+    // material order skip it, unless a guide trains on their records (which
+    // arrive in shading order); films are the same bits either way where the
     // scene has no layered materials (with them, the sorted bounces split
     // between two builds of the shading kernel). Measured device ms, sorted /
     // unsorted: one closure class, 1 M paths, 36 to 20,412 triangles 1.58 /
@@ -232,7 +233,7 @@ struct cenote_renderer {
     static constexpr uint32_t SORT_MIN_PATHS = 1u << 18;
     static constexpr uint32_t UNIFORM_MAX_TRIANGLES = 1u << 15;
     uint32_t sort_mode(const cenote_scene* sc, uint32_t paths) const {
-        if (sort_chosen || sc->ds.has_layers) return material_sort;
+        if (sort_chosen || sc->ds.has_layers || (guide && guide_steps > 0)) return material_sort;
         if (sc->uniform_shading || (paths != 0 && paths < SORT_MIN_PATHS)) return CENOTE_SORT_NONE;
         return material_sort;
     }
