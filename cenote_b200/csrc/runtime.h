@@ -63,11 +63,19 @@ struct DeviceBuffer {
         ptr = nullptr;
         bytes = 0;
     }
+    // A refused allocation leaves the buffer empty (`bytes` 0, so that a caller
+    // who keeps it by size asks again) and no error behind for the next launch.
     cudaError_t alloc(size_t n) {
         release();
         if (n == 0) n = 16;
+        const cudaError_t e = cudaMalloc(&ptr, n);
+        if (e != cudaSuccess) {
+            ptr = nullptr;
+            cudaGetLastError();
+            return e;
+        }
         bytes = n;
-        return cudaMalloc(&ptr, n);
+        return cudaSuccess;
     }
     template <class T>
     T* as() const {
