@@ -5,9 +5,11 @@
 #pragma once
 #include <atomic>
 #include <cstdint>
+#include <initializer_list>
 #include <memory>
 #include <mutex>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -82,6 +84,20 @@ struct DeviceBuffer {
         return static_cast<T*>(ptr);
     }
 };
+
+// Re-allocate buffers that grow together: all of them, or none is left (a
+// refused one gives the others back).
+inline cudaError_t alloc_together(std::initializer_list<std::pair<DeviceBuffer*, size_t>> buffers) {
+    for (const auto& b : buffers) b.first->release();
+    for (const auto& b : buffers) {
+        const cudaError_t e = b.first->alloc(b.second);
+        if (e != cudaSuccess) {
+            for (const auto& x : buffers) x.first->release();
+            return e;
+        }
+    }
+    return cudaSuccess;
+}
 
 }  // namespace cn
 
@@ -248,12 +264,19 @@ struct cenote_renderer {
 
     cudaError_t ensure(size_t cap) {
         if (cap <= pool_cap) return cudaSuccess;
-        cudaError_t e;
-        if ((e = ray.alloc(cap * 32)) || (e = flux.alloc(cap * 32)) || (e = hit.alloc(cap * 16)) ||
-            (e = ps.alloc(cap * 8)) || (e = q0.alloc(cap * 4)) || (e = q1.alloc(cap * 4)) ||
-            (e = shadows.alloc(cap * sizeof(ShadowRay))) || (e = shadow_queue.alloc(cap * 4)) || (e = sort_order.alloc(cap * 4)) ||
-            (e = sort_keys.alloc(cap * 4)) || (e = sort_bins.alloc(cn::SORT_BINS * 4)))
-            return e;
+        pool_cap = 0;
+        cudaError_t e = cn::alloc_together({{&ray, cap * 32},
+                                            {&flux, cap * 32},
+                                            {&hit, cap * 16},
+                                            {&ps, cap * 8},
+                                            {&q0, cap * 4},
+                                            {&q1, cap * 4},
+                                            {&shadows, cap * sizeof(ShadowRay)},
+                                            {&shadow_queue, cap * 4},
+                                            {&sort_order, cap * 4},
+                                            {&sort_keys, cap * 4},
+                                            {&sort_bins, cn::SORT_BINS * 4}});
+        if (e != cudaSuccess) return e;
         pool.ray = ray.as<float4>();
         pool.flux = flux.as<float4>();
         pool.hit = hit.as<uint4>();
@@ -275,15 +298,16 @@ struct cenote_renderer {
     // The learned guide's lanes, sized with the pool; detached without a guide.
     cudaError_t set_learned_guide(bool on) {
         if (on && g_cap < pool_cap) {
-            cudaError_t e;
-            if ((e = g_out.alloc(pool_cap * guide::OUT_ACT * 4)) || (e = g_rec.alloc(pool_cap * 4))) return e;
+            g_cap = 0;
+            cudaError_t e = cn::alloc_together({{&g_out, pool_cap * guide::OUT_ACT * 4}, {&g_rec, pool_cap * 4}});
+            if (e != cudaSuccess) return e;
             g_cap = pool_cap;
         }
         if (on && !g_records.ptr) {
-            cudaError_t e;
-            if ((e = g_records.alloc(size_t(GUIDE_RECORDS) * sizeof(guide::Record))) || (e = g_count.alloc(16)) ||
-                (e = g_sink.alloc(sizeof(GuideRecordSink))))
-                return e;
+            cudaError_t e = cn::alloc_together({{&g_records, size_t(GUIDE_RECORDS) * sizeof(guide::Record)},
+                                                {&g_count, 16},
+                                                {&g_sink, sizeof(GuideRecordSink)}});
+            if (e != cudaSuccess) return e;
         }
         pool.guide_out = on ? g_out.as<float>() : nullptr;
         pool.guide_rec = on ? g_rec.as<uint32_t>() : nullptr;
@@ -304,8 +328,9 @@ struct cenote_renderer {
 
         cudaError_t set_guides(bool on) {
         if (on && aov_cap < pool_cap) {
-            cudaError_t e;
-            if ((e = aov.alloc(pool_cap * 32)) || (e = aov_guide.alloc(pool_cap * 16))) return e;
+            aov_cap = 0;
+            cudaError_t e = cn::alloc_together({{&aov, pool_cap * 32}, {&aov_guide, pool_cap * 16}});
+            if (e != cudaSuccess) return e;
             aov_cap = pool_cap;
         }
         pool.aov = on ? aov.as<float4>() : nullptr;
@@ -332,13 +357,15 @@ struct cenote_guide {
     }
     cudaError_t ensure(size_t n) {
         if (n <= cap) return cudaSuccess;
-        cudaError_t e;
-        if ((e = feats.alloc(n * guide::IN * 4)) || (e = out.alloc(n * guide::OUT * 4)) ||
-            (e = save.alloc(n * guide::ACT * 2)) || (e = dz4.alloc(n * guide::OUT_PAD * 2)) ||
-            (e = dirs.alloc(n * 12)) || (e = weights.alloc(n * 4)))
-            return e;
-        cap = n;
-        return cudaSuccess;
+        cap = 0;
+        cudaError_t e = cn::alloc_together({{&feats, n * guide::IN * 4},
+                                            {&out, n * guide::OUT * 4},
+                                            {&save, n * guide::ACT * 2},
+                                            {&dz4, n * guide::OUT_PAD * 2},
+                                            {&dirs, n * 12},
+                                            {&weights, n * 4}});
+        if (e == cudaSuccess) cap = n;
+        return e;
     }
 };
 

@@ -211,6 +211,13 @@ void launch_light_leaves(const float4*, uint32_t, const GeomRecord*, uint32_t*, 
 }
 
 namespace guide {
+void launch_infer_paths(const Buffers&, const DeviceScene&, const PathPool& p, uint32_t, uint32_t n0, int,
+                        cudaStream_t) {
+    check(holds(p.guide_out, uint64_t(n0) * OUT_ACT * 4));
+}
+void launch_forward(const Buffers&, const float* feats, uint32_t rows, float* out, __nv_bfloat16*, int, cudaStream_t) {
+    check(holds(feats, uint64_t(rows) * IN * 4) && holds(out, uint64_t(rows) * OUT * 4));
+}
 void launch_resolve_records(Record* recs, const uint32_t* count, uint32_t capacity, const float4*, cudaStream_t) {
     check(holds(recs, uint64_t(capacity) * sizeof(Record)) && holds(count, 4));
 }

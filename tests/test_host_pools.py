@@ -39,7 +39,87 @@ def a_refused_one_shot_image(lib):
         assert lib.fake_bad_launches() == 0
 
 
-SCENARIOS = {f.__name__: f for f in (a_refused_one_shot_image,)}
+def refused_growth(lib, make, small, large):
+    """Refuse each allocation of a growth in turn: afterwards the small call, and
+    then the large one, run on buffers that are theirs."""
+    k = 0
+    while True:
+        state = make()
+        small(state)
+        lib.fake_refuse_after(k)
+        try:
+            large(state)
+        except Exception as e:
+            assert "out of memory" in str(e)
+        else:
+            break  # every allocation of the growth went through
+        small(state)
+        large(state)
+        assert lib.fake_bad_launches() == 0, k
+        k += 1
+    lib.fake_refuse_after(-1)
+    return k
+
+
+def a_refused_pool(lib):
+    from cenote_b200 import Context, Film, Guide, Renderer
+
+    ctx = Context(0)
+    scene = small_scene(ctx)
+    films = Film(ctx, 32, 32), Film(ctx, 200, 100)
+    guide = Guide(ctx, 1)
+
+    def call(film):
+        return lambda r: r.accumulate(scene, film, 2)
+
+    def guided():
+        r = Renderer(ctx, 2)
+        r.set_guide(guide, 0.5, 0)
+        return r
+
+    for make, fields in ((lambda: Renderer(ctx, 2), 13), (guided, 15)):
+        assert refused_growth(lib, make, call(films[0]), call(films[1])) >= fields
+
+
+def refused_guide_lanes(lib):
+    """The guide's lanes, refused on a pool that stays as it is."""
+    from cenote_b200 import Context, Film, Guide, Renderer
+
+    ctx = Context(0)
+    scene, film = small_scene(ctx), Film(ctx, 64, 64)
+    guide = Guide(ctx, 1)
+
+    def make():
+        r = Renderer(ctx, 2)
+        r.accumulate(scene, film, 1)
+        return r
+
+    def small(r):
+        r.set_guide(None)
+        r.accumulate(scene, film, 1)
+
+    def large(r):
+        r.set_guide(guide, 0.5, 0)
+        r.accumulate(scene, film, 1)
+
+    assert refused_growth(lib, make, small, large) >= 5
+
+
+def a_refused_guide_batch(lib):
+    import numpy as np
+
+    from cenote_b200 import Context, Guide
+
+    ctx = Context(0)
+
+    def forward(n):
+        return lambda g: g.forward(np.zeros((n, 96), np.float32))
+
+    assert refused_growth(lib, lambda: Guide(ctx, 1), forward(100), forward(1000)) >= 6
+
+
+SCENARIOS = {f.__name__: f for f in (a_refused_one_shot_image, a_refused_pool, refused_guide_lanes,
+                                     a_refused_guide_batch)}
 
 
 @pytest.mark.parametrize("name", SCENARIOS)
