@@ -1079,7 +1079,7 @@ int32_t run_waves(cenote_renderer* r, cenote_scene* sc, uint32_t width, uint32_t
     CN_CUDA(r->ensure_side());
     // Films trace the guides (Renderer::accumulate); one-shot renders do not.
     CN_CUDA(r->set_guides(film != nullptr));
-    CN_CUDA(r->set_learned_guide(r->guide != nullptr));
+    CN_CUDA(r->set_learned_guide(r->guide != nullptr, plan.need));
     if (r->guide) CN_CUDA(r->guide->ensure(cenote_renderer::GUIDE_BATCH));
 
     const bool timing = (r->profiling & CENOTE_PROFILE_TIMING) != 0;

@@ -295,13 +295,15 @@ struct cenote_renderer {
         return cudaSuccess;
     }
 
-    // The learned guide's lanes, sized with the pool; detached without a guide.
-    cudaError_t set_learned_guide(bool on) {
-        if (on && g_cap < pool_cap) {
+    // The learned guide's lanes for waves of `paths` paths (196 bytes each; a
+    // pool that unguided waves have grown is up to four times a guided wave);
+    // detached without a guide.
+    cudaError_t set_learned_guide(bool on, size_t paths) {
+        if (on && g_cap < paths) {
             g_cap = 0;
-            cudaError_t e = cn::alloc_together({{&g_out, pool_cap * guide::OUT_ACT * 4}, {&g_rec, pool_cap * 4}});
+            cudaError_t e = cn::alloc_together({{&g_out, paths * guide::OUT_ACT * 4}, {&g_rec, paths * 4}});
             if (e != cudaSuccess) return e;
-            g_cap = pool_cap;
+            g_cap = paths;
         }
         if (on && !g_records.ptr) {
             cudaError_t e = cn::alloc_together({{&g_records, size_t(GUIDE_RECORDS) * sizeof(guide::Record)},

@@ -118,8 +118,33 @@ def a_refused_guide_batch(lib):
     assert refused_growth(lib, lambda: Guide(ctx, 1), forward(100), forward(1000)) >= 6
 
 
+def guide_lanes_fit_the_guided_wave(lib):
+    """A guide attached after a large film takes the lanes of its own waves, not
+    of the pool that the film left."""
+    from cenote_b200 import Context, Film, Guide, Renderer
+
+    ctx = Context(0)
+    scene, film = small_scene(ctx), Film(ctx, 1024, 1024)
+    guide = Guide(ctx, 1)
+    taken = []
+    for samples in (0, 64):  # a fresh renderer, and one whose pool holds 2^26 paths
+        r = Renderer(ctx, 2)
+        if samples:
+            r.accumulate(scene, film, samples)
+            assert lib.fake_largest_wave() == 1 << 26
+        r.set_guide(guide, 0.5, 0)
+        r.accumulate(scene, film, 1)
+        before = lib.fake_live_bytes()
+        r.accumulate(scene, film, 64)
+        taken.append(lib.fake_live_bytes() - before)
+        r.close()
+        assert lib.fake_bad_launches() == 0
+    lanes = (15 << 20) * (48 * 4 + 4)  # 48 floats and a record index for 2^24 - 2^20 more paths
+    assert taken[1] == lanes < taken[0]
+
+
 SCENARIOS = {f.__name__: f for f in (a_refused_one_shot_image, a_refused_pool, refused_guide_lanes,
-                                     a_refused_guide_batch)}
+                                     a_refused_guide_batch, guide_lanes_fit_the_guided_wave)}
 
 
 @pytest.mark.parametrize("name", SCENARIOS)
