@@ -79,23 +79,33 @@ WavePlan plan_waves(const cenote_renderer* r, uint64_t pixels, uint32_t count, b
         // and 222 ms in waves of 16, 33 and 66 M paths, the chart's 56.6, 54.9
         // and 54.1 in waves of 17, 33 and 59 M. A guide that trains once per
         // wave keeps the 16 M of its schedule.
-        uint64_t paths = uint64_t(1) << 24;
-        if (!oneshot && !r->guide && pixels * count > paths) {
-            size_t free_bytes = 0, total = 0;
+        auto samples = [&](uint64_t paths) {
+            return uint32_t(std::max<uint64_t>(1, std::min<uint64_t>({paths / pixels, 64, count})));
+        };
+        p.spw = samples(uint64_t(1) << 24);
+        if (!oneshot && !r->guide) {
+            // Asked of the wave as it will be, in whole samples, and with the
+            // pool's own memory counted as free (growing gives it back first):
+            // the same call gets the same wave whatever the pool holds already.
+            uint64_t avail = 0;
             for (uint64_t big : {uint64_t(1) << 26, uint64_t(1) << 25}) {
-                const uint64_t need = std::min<uint64_t>(big, pixels * count);
-                if (need > r->pool_cap && !free_bytes && cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) {
-                    cudaGetLastError();
-                    break;
+                const uint32_t spw = samples(big);
+                const uint64_t need = pixels * spw;
+                if (spw <= p.spw) break;
+                if (need > r->pool_cap && !avail) {
+                    size_t free_bytes = 0, total = 0;
+                    if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) {
+                        cudaGetLastError();
+                        break;
+                    }
+                    avail = free_bytes + r->pool_cap * cenote_renderer::PATH_BYTES;
                 }
-                if (need <= r->pool_cap || need * cenote_renderer::PATH_BYTES <= free_bytes / 8) {
-                    paths = big;
+                if (need <= r->pool_cap || need * cenote_renderer::PATH_BYTES <= avail / 8) {
+                    p.spw = spw;
                     break;
                 }
             }
         }
-        uint64_t want = paths / pixels;
-        p.spw = uint32_t(std::max<uint64_t>(1, std::min<uint64_t>(want, 64)));
     }
     if (oneshot) p.spw = 1;
     p.spw = std::max(1u, std::min(p.spw, count));

@@ -143,8 +143,34 @@ def guide_lanes_fit_the_guided_wave(lib):
     assert taken[1] == lanes < taken[0]
 
 
+def the_same_call_gets_the_same_wave(lib):
+    """A film's waves do not shrink because the first call's pool took the memory
+    that the wave size was chosen by."""
+    from cenote_b200 import Context, Film, Renderer
+
+    ctx = Context(0)
+    scene = small_scene(ctx)
+    for gb in (300, 120, 100, 65, 50):
+        for w, h, n in ((1920, 1080, 64), (1280, 720, 64), (333, 217, 64), (5000, 4000, 3)):
+            lib.fake_limit(lib.fake_live_bytes() + (gb << 30))
+            r, film = Renderer(ctx, 2), Film(ctx, w, h)
+            waves = []
+            for k in range(3):
+                asked = lib.fake_meminfo_calls()
+                r.accumulate(scene, film, n)
+                waves.append(r.stats()["samples_per_wave"])
+                # Only a first call looks at the memory, unless it was refused the largest wave.
+                assert k == 0 or lib.fake_meminfo_calls() == asked or w * h * waves[k] < 1 << 25
+            assert waves[0] == waves[1] == waves[2], (gb, w, h, waves)
+            assert w * h * waves[0] <= 1 << 26
+            r.close()
+            film.close()
+    assert lib.fake_bad_launches() == 0
+
+
 SCENARIOS = {f.__name__: f for f in (a_refused_one_shot_image, a_refused_pool, refused_guide_lanes,
-                                     a_refused_guide_batch, guide_lanes_fit_the_guided_wave)}
+                                     a_refused_guide_batch, guide_lanes_fit_the_guided_wave,
+                                     the_same_call_gets_the_same_wave)}
 
 
 @pytest.mark.parametrize("name", SCENARIOS)
