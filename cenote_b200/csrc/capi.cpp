@@ -404,10 +404,10 @@ int32_t cenote_scene_create(cenote_context* ctx, const cenote_object* objects, u
     return cenote_scene_create_textured(ctx, objects, object_count, camera, env, deltas, delta_count, nullptr, 0, out);
 }
 
-int32_t cenote_scene_create_textured(cenote_context* ctx, const cenote_object* objects, uint32_t object_count,
-                                     const cenote_camera* camera, const cenote_environment* env,
-                                     const cenote_delta_light* deltas, uint32_t delta_count,
-                                     const cenote_texture* textures, uint32_t texture_count, cenote_scene** out) {
+static int32_t create_scene(cenote_context* ctx, const cenote_object* objects, uint32_t object_count,
+                            const cenote_camera* camera, const cenote_environment* env,
+                            const cenote_delta_light* deltas, uint32_t delta_count, const cenote_texture* textures,
+                            uint32_t texture_count, cenote_scene** out) {
     CN_CHECK(ctx && out, CENOTE_E_INVALID_ARGUMENT, "null context or output handle");
     *out = nullptr;
     CN_CHECK(objects && object_count > 0, CENOTE_E_INVALID_ARGUMENT, "a scene needs at least one object");
@@ -752,6 +752,15 @@ int32_t cenote_scene_create_textured(cenote_context* ctx, const cenote_object* o
     return CENOTE_OK;
 }
 
+int32_t cenote_scene_create_textured(cenote_context* ctx, const cenote_object* objects, uint32_t object_count,
+                                     const cenote_camera* camera, const cenote_environment* env,
+                                     const cenote_delta_light* deltas, uint32_t delta_count,
+                                     const cenote_texture* textures, uint32_t texture_count, cenote_scene** out) {
+    return creating(ctx, [&] {
+        return create_scene(ctx, objects, object_count, camera, env, deltas, delta_count, textures, texture_count, out);
+    });
+}
+
 void cenote_scene_destroy(cenote_scene* scene) {
     if (!scene) return;
     cenote_context* ctx = scene->ctx;
@@ -861,12 +870,18 @@ int32_t cenote_renderer_create(cenote_context* ctx, uint32_t max_bounces, uint32
     r->pool.counters = r->counters.as<uint32_t>();
     retain(ctx);
     *out = r.release();
+    std::lock_guard<std::mutex> list(ctx->renderers_mu);
+    ctx->renderers.push_back(*out);
     return CENOTE_OK;
 }
 
 void cenote_renderer_destroy(cenote_renderer* r) {
     if (!r) return;
     cenote_context* ctx = r->ctx;
+    {
+        std::lock_guard<std::mutex> list(ctx->renderers_mu);
+        ctx->renderers.erase(std::remove(ctx->renderers.begin(), ctx->renderers.end(), r), ctx->renderers.end());
+    }
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
     delete r;
@@ -962,24 +977,26 @@ int32_t cenote_film_create(cenote_context* ctx, uint32_t width, uint32_t height,
     *out = nullptr;
     CN_CHECK(width > 0 && height > 0, CENOTE_E_INVALID_ARGUMENT, "zero-sized film");
     CN_CHECK(uint64_t(width) * height < (1ull << 31), CENOTE_E_INVALID_ARGUMENT, "film too large");
-    CN_CUDA(cudaSetDevice(ctx->device));
-    auto f = std::make_unique<cenote_film>();
-    f->ctx = ctx;
-    f->width = width;
-    f->height = height;
-    size_t px = size_t(width) * height;
-    CN_CUDA(f->sum.alloc(px * 16));
-    CN_CUDA(f->avg.alloc(px * 16));
-    CN_CUDA(f->albedo.alloc(px * 16));
-    CN_CUDA(f->normal.alloc(px * 16));
-    CN_CUDA(f->depth.alloc(px * 4));
-    CN_CUDA(cudaMemsetAsync(f->sum.ptr, 0, px * 16, ctx->stream));
-    CN_CUDA(cudaMemsetAsync(f->albedo.ptr, 0, px * 16, ctx->stream));
-    CN_CUDA(cudaMemsetAsync(f->normal.ptr, 0, px * 16, ctx->stream));
-    CN_CUDA(cudaMemsetAsync(f->depth.ptr, 0, px * 4, ctx->stream));
-    retain(ctx);
-    *out = f.release();
-    return CENOTE_OK;
+    return creating(ctx, [&]() -> int32_t {
+        CN_CUDA(cudaSetDevice(ctx->device));
+        auto f = std::make_unique<cenote_film>();
+        f->ctx = ctx;
+        f->width = width;
+        f->height = height;
+        size_t px = size_t(width) * height;
+        CN_CUDA(f->sum.alloc(px * 16));
+        CN_CUDA(f->avg.alloc(px * 16));
+        CN_CUDA(f->albedo.alloc(px * 16));
+        CN_CUDA(f->normal.alloc(px * 16));
+        CN_CUDA(f->depth.alloc(px * 4));
+        CN_CUDA(cudaMemsetAsync(f->sum.ptr, 0, px * 16, ctx->stream));
+        CN_CUDA(cudaMemsetAsync(f->albedo.ptr, 0, px * 16, ctx->stream));
+        CN_CUDA(cudaMemsetAsync(f->normal.ptr, 0, px * 16, ctx->stream));
+        CN_CUDA(cudaMemsetAsync(f->depth.ptr, 0, px * 4, ctx->stream));
+        retain(ctx);
+        *out = f.release();
+        return CENOTE_OK;
+    });
 }
 
 void cenote_film_destroy(cenote_film* film) {
@@ -1075,12 +1092,22 @@ int32_t run_waves(cenote_renderer* r, cenote_scene* sc, uint32_t width, uint32_t
     const uint64_t pixels = uint64_t(width) * height;
     WavePlan plan = plan_waves(r, pixels, count, oneshot != nullptr);
     CN_CHECK(plan.need < (1ull << 31), CENOTE_E_INVALID_ARGUMENT, "wave too large");
-    CN_CUDA(r->ensure(plan.need));
     CN_CUDA(r->ensure_side());
-    // Films trace the guides (Renderer::accumulate); one-shot renders do not.
-    CN_CUDA(r->set_guides(film != nullptr));
-    CN_CUDA(r->set_learned_guide(r->guide != nullptr, plan.need));
-    if (r->guide) CN_CUDA(r->guide->ensure(cenote_renderer::GUIDE_BATCH));
+    auto allocate = [&] {
+        cudaError_t e = r->ensure(plan.need);
+        // Films trace the guides (Renderer::accumulate); one-shot renders do not.
+        if (e == cudaSuccess) e = r->set_guides(film != nullptr);
+        if (e == cudaSuccess) e = r->set_learned_guide(r->guide != nullptr, plan.need);
+        if (e == cudaSuccess && r->guide) e = r->guide->ensure(cenote_renderer::GUIDE_BATCH);
+        return e;
+    };
+    cudaError_t e = allocating(ctx, allocate);
+    if (e == cudaErrorMemoryAllocation && plan.need > cenote_renderer::PLAIN_WAVE) {
+        r->release_pool();  // the memory was there a moment ago: a plain wave then
+        plan = plan_waves(r, pixels, count, oneshot != nullptr, cenote_renderer::PLAIN_WAVE);
+        e = allocate();
+    }
+    CN_CUDA(e);
 
     const bool timing = (r->profiling & CENOTE_PROFILE_TIMING) != 0;
     const bool counting = (r->profiling & CENOTE_PROFILE_COUNTS) != 0;
@@ -1275,7 +1302,7 @@ int32_t cenote_render_once(cenote_renderer* r, cenote_scene* scene, uint32_t wid
     std::lock_guard<std::mutex> lock(r->ctx->mu);
     CN_CUDA(cudaSetDevice(r->ctx->device));
     const size_t bytes = size_t(width) * height * 16;
-    if (r->oneshot.bytes < bytes) CN_CUDA(r->oneshot.alloc(bytes));
+    if (r->oneshot.bytes < bytes) CN_CUDA(allocating(r->ctx, [&] { return r->oneshot.alloc(bytes); }));
     int32_t rc = run_waves(r, scene, width, height, sample, 1, nullptr, r->oneshot.as<float4>());
     if (rc != CENOTE_OK) return rc;
     return copy_out(r->ctx, rgba_out, r->oneshot.ptr, bytes);

@@ -117,7 +117,7 @@ int32_t cenote_guide_forward(cenote_guide* g, const float* feats, uint32_t n, fl
     if (n == 0) return CENOTE_OK;
     std::lock_guard<std::mutex> lock(g->ctx->mu);
     CN_CUDA(cudaSetDevice(g->ctx->device));
-    CN_CUDA(g->ensure(n));
+    CN_CUDA(allocating(g->ctx, [&] { return g->ensure(n); }));
     cudaStream_t s = g->ctx->stream;
     CN_CUDA(cudaMemcpyAsync(g->feats.ptr, feats, size_t(n) * guide::IN * 4, cudaMemcpyHostToDevice, s));
     guide::launch_forward(g->view(), g->feats.as<float>(), n, g->out.as<float>(), nullptr, g->sms, s);
@@ -133,7 +133,7 @@ int32_t cenote_guide_train_step(cenote_guide* g, const float* feats, const float
     CN_CHECK(n > 0, CENOTE_E_INVALID_ARGUMENT, "empty batch");
     std::lock_guard<std::mutex> lock(g->ctx->mu);
     CN_CUDA(cudaSetDevice(g->ctx->device));
-    CN_CUDA(g->ensure(n));
+    CN_CUDA(allocating(g->ctx, [&] { return g->ensure(n); }));
     cudaStream_t s = g->ctx->stream;
     CN_CUDA(cudaMemcpyAsync(g->feats.ptr, feats, size_t(n) * guide::IN * 4, cudaMemcpyHostToDevice, s));
     CN_CUDA(cudaMemcpyAsync(g->dirs.ptr, dirs, size_t(n) * 12, cudaMemcpyHostToDevice, s));

@@ -62,8 +62,19 @@ int32_t copy_out(cenote_context* ctx, void* host, const void* device, size_t byt
     return wait_stream(ctx->stream, ctx->sync_ev, 600000.0);
 }
 
+bool give_back_pools(cenote_context* ctx) {
+    std::lock_guard<std::mutex> list(ctx->renderers_mu);
+    bool any = false;
+    for (cenote_renderer* r : ctx->renderers)
+        if (r->pool_cap > cenote_renderer::PLAIN_WAVE) {
+            r->release_pool();
+            any = true;
+        }
+    return any;
+}
+
 // How a call splits into waves: `range` pixels per wave, `spw` samples each.
-WavePlan plan_waves(const cenote_renderer* r, uint64_t pixels, uint32_t count, bool oneshot) {
+WavePlan plan_waves(const cenote_renderer* r, uint64_t pixels, uint32_t count, bool oneshot, uint64_t most) {
     WavePlan p{uint32_t(pixels), 1, 0};
     if (r->capacity_req && r->capacity_req < pixels) {
         p.range = r->capacity_req;
@@ -82,13 +93,13 @@ WavePlan plan_waves(const cenote_renderer* r, uint64_t pixels, uint32_t count, b
         auto samples = [&](uint64_t paths) {
             return uint32_t(std::max<uint64_t>(1, std::min<uint64_t>({paths / pixels, 64, count})));
         };
-        p.spw = samples(uint64_t(1) << 24);
+        p.spw = samples(cenote_renderer::PLAIN_WAVE);
         if (!oneshot && !r->guide) {
             // Asked of the wave as it will be, in whole samples, and with the
             // pool's own memory counted as free (growing gives it back first):
             // the same call gets the same wave whatever the pool holds already.
             uint64_t avail = 0;
-            for (uint64_t big : {uint64_t(1) << 26, uint64_t(1) << 25}) {
+            for (uint64_t big : {most, most / 2}) {
                 const uint32_t spw = samples(big);
                 const uint64_t need = pixels * spw;
                 if (spw <= p.spw) break;

@@ -111,6 +111,8 @@ using cn::FilmTargets;
 using cn::GuideRecordSink;
 namespace guide = cn::guide;
 
+struct cenote_renderer;
+
 struct cenote_context {
     // Handles made from this context hold a reference; the context is freed
     // when cenote_context_destroy has been called and the last one is gone,
@@ -123,6 +125,9 @@ struct cenote_context {
     LaunchShape shape{};
     cn::DeviceBuffer tables;
     std::mutex mu;
+    // The renderers made from this context, for give_back_pools.
+    std::mutex renderers_mu;
+    std::vector<cenote_renderer*> renderers;
     unsigned long long* tally_host = nullptr;  // pinned: a wave's counters come back with its last event
     // L2 persistence (this context's own set-aside; nothing outlives it).
     size_t l2_persist_max = 0, l2_window_max = 0, l2_set_aside = 0;
@@ -211,6 +216,8 @@ struct cenote_renderer {
     size_t g_cap = 0;
     // Device bytes a path of the pool takes with the denoiser guides' lanes.
     static constexpr uint64_t PATH_BYTES = 32 * 2 + 16 + 8 + 8 + sizeof(ShadowRay) + 4 + 8 + 48;
+    // Waves above this many paths are taken only while memory is plentiful.
+    static constexpr uint64_t PLAIN_WAVE = uint64_t(1) << 24;
     static constexpr uint32_t GUIDE_RECORDS = 1u << 20;
     static constexpr uint32_t GUIDE_BATCH = 65536;
     // The shadow walks' own stream and the events that fork it off the main
@@ -260,6 +267,14 @@ struct cenote_renderer {
         if (sort_chosen || sc->ds.has_layers || (guide && guide_steps > 0)) return material_sort;
         if (sc->uniform_shading || (paths != 0 && paths < SORT_MIN_PATHS)) return CENOTE_SORT_NONE;
         return material_sort;
+    }
+
+    // Free the pool and every lane sized by a wave (not the one-shot image); the next wave allocates anew.
+    void release_pool() {
+        pool_cap = aov_cap = g_cap = 0;
+        for (DeviceBuffer* b : {&ray, &flux, &hit, &ps, &q0, &q1, &shadows, &shadow_queue, &sort_order, &sort_keys,
+                                &sort_bins, &aov, &aov_guide, &g_out, &g_rec})
+            b->release();
     }
 
     cudaError_t ensure(size_t cap) {
@@ -403,6 +418,32 @@ inline void release(cenote_context* ctx) {
 
 namespace cn {
 
+// Free the pools of the context's renderers that are larger than a plain wave's
+// (they were taken because memory was plentiful). True when any was. The
+// caller holds ctx->mu, so no wave of the context is in flight.
+bool give_back_pools(cenote_context* ctx);
+
+// Allocations under ctx->mu: refused, they are tried once more if large pools
+// could be given back.
+template <class F>
+cudaError_t allocating(cenote_context* ctx, F allocations) {
+    const cudaError_t e = allocations();
+    return e == cudaErrorMemoryAllocation && give_back_pools(ctx) ? allocations() : e;
+}
+
+// The same for a call that makes a new object and leaves nothing behind when
+// it is refused; ctx->mu is not held.
+template <class F>
+int32_t creating(cenote_context* ctx, F call) {
+    const int32_t rc = call();
+    if (rc != CENOTE_E_ALLOCATION) return rc;
+    {
+        std::lock_guard<std::mutex> lock(ctx->mu);
+        if (!give_back_pools(ctx)) return rc;
+    }
+    return call();
+}
+
 // How a call splits into waves: `range` pixels per wave, `spw` samples each.
 struct WavePlan {
     uint32_t range, spw;
@@ -414,7 +455,9 @@ struct WaveCounts {
     size_t events = 0;
 };
 
-WavePlan plan_waves(const cenote_renderer* r, uint64_t pixels, uint32_t count, bool oneshot);
+// An automatic wave takes at most `most` paths where whole samples allow.
+WavePlan plan_waves(const cenote_renderer* r, uint64_t pixels, uint32_t count, bool oneshot,
+                    uint64_t most = uint64_t(1) << 26);
 
 // Enqueue `count` samples from `sample0` for every pixel on `stream`, with no
 // host synchronisation (so a stream capture can record it): each wave's

@@ -303,8 +303,19 @@ struct cenote_server {
                 if (used + cached + bytes + scene_bytes > budget) break;
             }
             queue.pop_front();
-            cudaError_t e;
-            if ((e = take_dev(j.sum, px * 16)) || (e = take_dev(j.avg, px * 16)) || (e = take_host(&j.host, px * 16))) {
+            auto take = [&] {
+                cudaError_t e = cudaSuccess;
+                if (!j.sum.ptr) e = take_dev(j.sum, px * 16);
+                if (e == cudaSuccess && !j.avg.ptr) e = take_dev(j.avg, px * 16);
+                if (e == cudaSuccess && !j.host) e = take_host(&j.host, px * 16);
+                return e;
+            };
+            cudaError_t e = take();
+            if (e == cudaErrorMemoryAllocation) {
+                std::lock_guard<std::mutex> lock(ctx->mu);
+                if (give_back_pools(ctx)) e = take();
+            }
+            if (e != cudaSuccess) {
                 j.free_device();
                 j.error = e == cudaErrorMemoryAllocation ? CENOTE_E_ALLOCATION : CENOTE_E_DEVICE;
                 j.state = CENOTE_JOB_FAILED;
@@ -672,7 +683,10 @@ int32_t cenote_server_create(cenote_context* ctx, uint64_t hbm_budget, const cen
         cenote_renderer& r = s->renderers[k];
         r.ctx = ctx;
         r.light_sampling = s->opt.light_sampling;
-        CN_CUDA(r.ensure(s->opt.pool_paths));
+        {
+            std::lock_guard<std::mutex> lock(ctx->mu);
+            CN_CUDA(allocating(ctx, [&] { return r.ensure(s->opt.pool_paths); }));
+        }
         CN_CUDA(r.counters.alloc(CTR_COUNT * 4));
         CN_CUDA(r.tally.alloc(64));
         CN_CUDA(cudaMemset(r.tally.ptr, 0, 64));

@@ -58,6 +58,6 @@ def main(scenarios: dict) -> None:
     for name in ("live_bytes", "meminfo_calls", "bad_launches", "windowed_walks", "window_free_shadows",
                  "open_windows", "bytes_at_leaves", "waves", "largest_wave"):
         getattr(lib, "fake_" + name).restype = ctypes.c_uint64
-    lib.fake_limit.argtypes = [ctypes.c_uint64]
+    lib.fake_limit.argtypes = lib.fake_refuse_above.argtypes = [ctypes.c_uint64]
     lib.fake_clock_ms.restype = ctypes.c_double
     scenarios[sys.argv[2]](lib)

@@ -48,6 +48,7 @@ extern "C" {
 
 void fake_limit(uint64_t bytes) { limit = bytes; }
 void fake_refuse_after(int n) { refuse_after = n; }
+void fake_refuse_above(uint64_t bytes) { refused_size = bytes; }
 void fake_hang(int on) { hang = on != 0; }
 uint64_t fake_live_bytes() { return live_bytes; }
 uint64_t fake_meminfo_calls() { return meminfo_calls; }
@@ -68,7 +69,7 @@ double fake_clock_ms() { return std::chrono::duration<double, std::milli>(clock_
 
 cudaError_t cudaMalloc(void** p, size_t n) {
     std::lock_guard<std::mutex> lock(mu);
-    if (refuse_after == 0 || live_bytes + n > limit) {
+    if (refuse_after == 0 || n > refused_size || live_bytes + n > limit) {
         refuse_after = -1;
         *p = nullptr;
         return last_error = cudaErrorMemoryAllocation;

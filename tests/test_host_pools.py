@@ -168,9 +168,62 @@ def the_same_call_gets_the_same_wave(lib):
     assert lib.fake_bad_launches() == 0
 
 
+def large_pools_are_given_back(lib):
+    """What does not fit beside a renderer's large pool gets its memory: the pool
+    was taken because memory was plentiful."""
+    import numpy as np
+
+    from cenote_b200 import Context, Film, Guide, Renderer, Server
+
+    ctx = Context(0)
+    scene, film, guide = small_scene(ctx), Film(ctx, 1024, 1024), Guide(ctx, 1)
+    other, image = Renderer(ctx, 2), Film(ctx, 640, 360)
+    kept = []
+
+    for call in (lambda: kept.append(Film(ctx, 3000, 2000)), lambda: kept.append(small_scene(ctx)),
+                 lambda: other.accumulate(scene, image, 4), lambda: other.render(scene, 1000, 700),
+                 lambda: guide.forward(np.zeros((50000, 96), np.float32)),
+                 lambda: kept.append(Server(ctx, 40 << 30, pool_paths=1 << 20))):
+        lib.fake_limit(lib.fake_live_bytes() + (200 << 30))
+        r = Renderer(ctx, 2)
+        film.reset()
+        r.accumulate(scene, film, 64)
+        assert r.stats()["samples_per_wave"] == 64
+        lib.fake_limit(lib.fake_live_bytes() + 1000)  # nothing of any size fits
+        call()
+        film.reset()
+        r.accumulate(scene, film, 64)  # and the renderer carries on, in smaller waves
+        assert r.stats()["samples_per_wave"] == 16
+        assert lib.fake_bad_launches() == 0
+        r.close()
+    for o in kept:
+        o.close()
+
+
+def a_refused_large_wave_is_a_plain_one(lib):
+    """Memory that the device reports free but does not give: the call runs in
+    waves of 2^24 paths, then and later."""
+    from cenote_b200 import Context, Film, Renderer
+
+    ctx = Context(0)
+    scene, film = small_scene(ctx), Film(ctx, 1024, 1024)
+    # The shadow records are a wave's largest field, 64 bytes a path: the large wave is
+    # refused from its first field on, or there.
+    for above in (64 << 24, 63 << 26):
+        lib.fake_refuse_above(above)
+        r = Renderer(ctx, 2)
+        for k in range(2):
+            film.reset()
+            r.accumulate(scene, film, 64)
+            assert r.stats()["samples_per_wave"] == 16
+        assert lib.fake_bad_launches() == 0
+        r.close()
+
+
 SCENARIOS = {f.__name__: f for f in (a_refused_one_shot_image, a_refused_pool, refused_guide_lanes,
                                      a_refused_guide_batch, guide_lanes_fit_the_guided_wave,
-                                     the_same_call_gets_the_same_wave)}
+                                     the_same_call_gets_the_same_wave, large_pools_are_given_back,
+                                     a_refused_large_wave_is_a_plain_one)}
 
 
 @pytest.mark.parametrize("name", SCENARIOS)
