@@ -89,12 +89,13 @@ WavePlan plan_waves(const cenote_renderer* r, uint64_t pixels, uint32_t count, b
         // 16 M (3.6 GB) in any case. The terrain's 64-spp frame takes 238, 228
         // and 222 ms in waves of 16, 33 and 66 M paths, the chart's 56.6, 54.9
         // and 54.1 in waves of 17, 33 and 59 M. A guide that trains once per
-        // wave keeps the 16 M of its schedule.
+        // wave keeps the 16 M of its schedule, and so does a renderer whose
+        // caller bounded its paths.
         auto samples = [&](uint64_t paths) {
             return uint32_t(std::max<uint64_t>(1, std::min<uint64_t>({paths / pixels, 64, count})));
         };
         p.spw = samples(cenote_renderer::PLAIN_WAVE);
-        if (!oneshot && !r->guide) {
+        if (!oneshot && !r->guide && !r->capacity_req) {
             // Asked of the wave as it will be, in whole samples, and with the
             // pool's own memory counted as free (growing gives it back first):
             // the same call gets the same wave whatever the pool holds already.

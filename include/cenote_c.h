@@ -266,8 +266,13 @@ int32_t cenote_scene_env_tables(cenote_scene* scene, float* marginal, float* con
 
 /* ---- renderer (Renderer::with_max_bounces, render/mod.rs:151) ----------------- */
 
-/* capacity = paths in flight per wave (0 = one full sample of the largest
- * target seen, grown on demand). */
+/* capacity: below an image's pixel count, the pixels a wave carries (one
+ * sample each); above it, waves take whole samples of the image, up to 2^24
+ * paths (3.7 GB of path state) or one sample if that is more. 0: the same, but
+ * up to 2^26 paths (14.8 GB) while an eighth of the free device memory holds
+ * them. The path state grows on demand and stays with the renderer; what is
+ * above 2^24 paths is given back when another allocation of the context is
+ * refused. */
 int32_t cenote_renderer_create(cenote_context* ctx, uint32_t max_bounces, uint32_t light_sampling,
                                uint32_t capacity, cenote_renderer** out);
 void cenote_renderer_destroy(cenote_renderer* r);

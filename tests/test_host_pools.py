@@ -220,10 +220,27 @@ def a_refused_large_wave_is_a_plain_one(lib):
         r.close()
 
 
+def a_capacity_bounds_the_waves(lib):
+    """A renderer made with a capacity keeps to waves of 2^24 paths."""
+    from cenote_b200 import Context, Film, Renderer
+
+    ctx = Context(0)
+    scene, film = small_scene(ctx), Film(ctx, 1024, 1024)
+    for capacity, samples, wave in ((0, 64, 1 << 26), (1 << 20, 16, 1 << 24), (3 << 20, 16, 1 << 24),
+                                    (1 << 27, 16, 1 << 24), (1000, 1, 1000)):
+        r = Renderer(ctx, 2, capacity=capacity)
+        waves = lib.fake_waves()
+        film.reset()
+        r.accumulate(scene, film, 64 if capacity != 1000 else 1)
+        assert r.stats()["samples_per_wave"] == samples, capacity
+        assert lib.fake_waves() - waves == -(-(64 << 20 if capacity != 1000 else 1 << 20) // wave), capacity
+        r.close()
+
+
 SCENARIOS = {f.__name__: f for f in (a_refused_one_shot_image, a_refused_pool, refused_guide_lanes,
                                      a_refused_guide_batch, guide_lanes_fit_the_guided_wave,
                                      the_same_call_gets_the_same_wave, large_pools_are_given_back,
-                                     a_refused_large_wave_is_a_plain_one)}
+                                     a_refused_large_wave_is_a_plain_one, a_capacity_bounds_the_waves)}
 
 
 @pytest.mark.parametrize("name", SCENARIOS)
