@@ -1032,7 +1032,8 @@ namespace {
 // enqueue on the context's stream, wait, then fold the counters and stage
 // timings into the renderer's stats.
 // While alive, the scene's wide BVH nodes are a persisting access-policy
-// window on the context's stream: the waves' streaming path state does not
+// window on the streams of the renderer's waves (the context's, and the side
+// stream of the shadow walks): the waves' streaming path state does not
 // evict them from L2. The window is cleared on exit; the persisting lines
 // (a device-wide state) are released once no window of this process is
 // active on the device, so a renderer finishing does not evict the window
@@ -1041,9 +1042,9 @@ std::mutex g_l2_mutex;
 int g_l2_active[64] = {};
 
 struct L2Window {
-    cudaStream_t stream = nullptr;
+    cudaStream_t streams[2] = {nullptr, nullptr};
     int device = -1;
-    L2Window(cenote_context* ctx, const cenote_scene* sc, bool on) {
+    L2Window(cenote_context* ctx, const cenote_scene* sc, cudaStream_t side, bool on) {
         const size_t bytes = std::min(size_t(sc->ds.node_count) * sizeof(WideNode), ctx->l2_window_max);
         if (!on || bytes == 0 || ctx->l2_persist_max == 0) return;
         const size_t want = std::min(bytes, ctx->l2_persist_max);
@@ -1060,22 +1061,22 @@ struct L2Window {
         a.accessPolicyWindow.hitRatio = std::min(1.0f, float(ctx->l2_set_aside) / float(bytes));
         a.accessPolicyWindow.hitProp = cudaAccessPropertyPersisting;
         a.accessPolicyWindow.missProp = cudaAccessPropertyStreaming;
-        if (cudaStreamSetAttribute(ctx->stream, cudaStreamAttributeAccessPolicyWindow, &a) == cudaSuccess) {
-            stream = ctx->stream;
-            if (ctx->device >= 0 && ctx->device < 64) {
-                device = ctx->device;
-                std::lock_guard<std::mutex> lock(g_l2_mutex);
-                g_l2_active[device]++;
-            }
-        } else {
-            cudaGetLastError();
+        int set = 0;
+        for (cudaStream_t s : {ctx->stream, side})
+            if (cudaStreamSetAttribute(s, cudaStreamAttributeAccessPolicyWindow, &a) == cudaSuccess) streams[set++] = s;
+            else cudaGetLastError();
+        if (set && ctx->device >= 0 && ctx->device < 64) {
+            device = ctx->device;
+            std::lock_guard<std::mutex> lock(g_l2_mutex);
+            g_l2_active[device]++;
         }
     }
     ~L2Window() {
-        if (!stream) return;
+        if (!streams[0]) return;
         cudaStreamAttrValue a{};
         a.accessPolicyWindow.num_bytes = 0;
-        cudaStreamSetAttribute(stream, cudaStreamAttributeAccessPolicyWindow, &a);
+        for (cudaStream_t s : streams)
+            if (s) cudaStreamSetAttribute(s, cudaStreamAttributeAccessPolicyWindow, &a);
         bool last = true;
         if (device >= 0) {
             std::lock_guard<std::mutex> lock(g_l2_mutex);
@@ -1088,11 +1089,11 @@ struct L2Window {
 int32_t run_waves(cenote_renderer* r, cenote_scene* sc, uint32_t width, uint32_t height, uint32_t sample0,
                   uint32_t count, cenote_film* film, float4* oneshot) {
     cenote_context* ctx = r->ctx;
-    L2Window l2(ctx, sc, r->l2_window != 0);
+    CN_CUDA(r->ensure_side());
+    L2Window l2(ctx, sc, r->side, r->l2_window != 0);
     const uint64_t pixels = uint64_t(width) * height;
     WavePlan plan = plan_waves(r, pixels, count, oneshot != nullptr);
     CN_CHECK(plan.need < (1ull << 31), CENOTE_E_INVALID_ARGUMENT, "wave too large");
-    CN_CUDA(r->ensure_side());
     auto allocate = [&] {
         cudaError_t e = r->ensure(plan.need);
         // Films trace the guides (Renderer::accumulate); one-shot renders do not.

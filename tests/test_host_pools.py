@@ -237,10 +237,34 @@ def a_capacity_bounds_the_waves(lib):
         r.close()
 
 
+def the_l2_window_covers_every_walk(lib):
+    """With the L2 window on, the shadow walks' stream carries it as well as the
+    closest-hit walks', and none is left when the call returns."""
+    from cenote_b200 import PROFILE_TIMING, Context, Film, Renderer
+
+    ctx = Context(0)
+    scene, film = small_scene(ctx), Film(ctx, 64, 64)
+    for flags in (0, PROFILE_TIMING):
+        r = Renderer(ctx, 4)
+        r.set_profiling(flags)
+        r.accumulate(scene, film, 2)
+        assert lib.fake_windowed_walks() == (0 if flags == 0 else 7)
+        shadows = lib.fake_window_free_shadows()
+        r.set_tuning(1, l2_window=1)
+        r.accumulate(scene, film, 2)
+        assert lib.fake_window_free_shadows() == shadows
+        assert lib.fake_windowed_walks() == (7 if flags == 0 else 14)  # 4 closest-hit and 3 shadow walks
+        assert lib.fake_open_windows() == 0
+        r.set_tuning(1)
+        r.accumulate(scene, film, 2)
+        assert lib.fake_window_free_shadows() == shadows + 3
+
+
 SCENARIOS = {f.__name__: f for f in (a_refused_one_shot_image, a_refused_pool, refused_guide_lanes,
                                      a_refused_guide_batch, guide_lanes_fit_the_guided_wave,
                                      the_same_call_gets_the_same_wave, large_pools_are_given_back,
-                                     a_refused_large_wave_is_a_plain_one, a_capacity_bounds_the_waves)}
+                                     a_refused_large_wave_is_a_plain_one, a_capacity_bounds_the_waves,
+                                     the_l2_window_covers_every_walk)}
 
 
 @pytest.mark.parametrize("name", SCENARIOS)
