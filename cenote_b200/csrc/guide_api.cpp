@@ -122,7 +122,7 @@ int32_t cenote_guide_forward(cenote_guide* g, const float* feats, uint32_t n, fl
     CN_CUDA(cudaMemcpyAsync(g->feats.ptr, feats, size_t(n) * guide::IN * 4, cudaMemcpyHostToDevice, s));
     guide::launch_forward(g->view(), g->feats.as<float>(), n, g->out.as<float>(), nullptr, g->sms, s);
     CN_CUDA(cudaGetLastError());
-    int32_t rc = copy_out(g->ctx, out, g->out.ptr, size_t(n) * guide::OUT * 4);
+    int32_t rc = copy_out(g->ctx, out, g->out.ptr, size_t(n) * guide::OUT * 4, 60000.0);
     if (rc != CENOTE_OK) return rc;
     return check_err(g);
 }

@@ -57,9 +57,9 @@ int32_t wait_event(cudaEvent_t ev, double timeout_ms) {
     }
 }
 
-int32_t copy_out(cenote_context* ctx, void* host, const void* device, size_t bytes) {
+int32_t copy_out(cenote_context* ctx, void* host, const void* device, size_t bytes, double timeout_ms) {
     CN_CUDA(cudaMemcpyAsync(host, device, bytes, cudaMemcpyDeviceToHost, ctx->stream));
-    return wait_stream(ctx->stream, ctx->sync_ev, 600000.0);
+    return wait_stream(ctx->stream, ctx->sync_ev, timeout_ms);
 }
 
 bool give_back_pools(cenote_context* ctx) {

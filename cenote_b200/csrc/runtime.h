@@ -50,8 +50,9 @@ const char* last_error();
 int32_t wait_stream(cudaStream_t s, cudaEvent_t ev, double timeout_ms);
 int32_t wait_event(cudaEvent_t ev, double timeout_ms);
 
-// Device memory to the caller's host memory on the context's stream, waited for.
-int32_t copy_out(cenote_context* ctx, void* host, const void* device, size_t bytes);
+// Device memory to the caller's host memory on the context's stream, waited for
+// as long as the work before it may take.
+int32_t copy_out(cenote_context* ctx, void* host, const void* device, size_t bytes, double timeout_ms = 600000.0);
 
 struct DeviceBuffer {
     void* ptr = nullptr;

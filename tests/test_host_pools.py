@@ -260,11 +260,33 @@ def the_l2_window_covers_every_walk(lib):
         assert lib.fake_window_free_shadows() == shadows + 3
 
 
+def waits_keep_their_bounds(lib):
+    """Work that never ends is reported after the call's own bound: a minute for
+    the guide's calls, ten for a render's."""
+    import numpy as np
+
+    from cenote_b200 import CenoteError, Context, Film, Guide, Renderer
+
+    ctx = Context(0)
+    scene, film, guide, r = small_scene(ctx), Film(ctx, 16, 16), Guide(ctx, 1), Renderer(ctx, 2)
+    feats, dirs = np.zeros((10, 96), np.float32), np.ones((10, 3), np.float32)
+    for bound, call in ((60, lambda: guide.forward(feats)),
+                        (60, lambda: guide.train_step(feats, dirs, np.ones(10, np.float32), 0.0)),
+                        (600, lambda: r.accumulate(scene, film, 1)), (600, lambda: film.averages()),
+                        (600, lambda: film.sums())):
+        lib.fake_hang(1)
+        before = lib.fake_clock_ms()
+        with pytest.raises(CenoteError, match="did not finish"):
+            call()
+        lib.fake_hang(0)
+        assert bound <= (lib.fake_clock_ms() - before) / 1e3 <= bound + 1
+
+
 SCENARIOS = {f.__name__: f for f in (a_refused_one_shot_image, a_refused_pool, refused_guide_lanes,
                                      a_refused_guide_batch, guide_lanes_fit_the_guided_wave,
                                      the_same_call_gets_the_same_wave, large_pools_are_given_back,
                                      a_refused_large_wave_is_a_plain_one, a_capacity_bounds_the_waves,
-                                     the_l2_window_covers_every_walk)}
+                                     the_l2_window_covers_every_walk, waits_keep_their_bounds)}
 
 
 @pytest.mark.parametrize("name", SCENARIOS)
