@@ -591,7 +591,7 @@ class Film:
             pass
 
 
-SORT_NONE, SORT_ALL, SORT_SECONDARY = 0, 1, 2
+SORT_NONE, SORT_ALL, SORT_SECONDARY, SORT_AUTO = 0, 1, 2, 0xFFFFFFFF
 
 
 class Renderer:
@@ -616,7 +616,8 @@ class Renderer:
         _check(library().cenote_renderer_set_samples_per_wave(self._h, n))
 
     def set_material_sort(self, mode: int) -> None:
-        """SORT_NONE, SORT_ALL or SORT_SECONDARY: shade each bounce's paths in material order."""
+        """SORT_NONE, SORT_ALL or SORT_SECONDARY: shade each bounce's paths in material order
+        (SORT_AUTO, a new renderer's: the waves that gain by it)."""
         _check(library().cenote_renderer_set_material_sort(self._h, mode))
 
     def tuning(self) -> dict:

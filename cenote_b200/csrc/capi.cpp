@@ -909,9 +909,8 @@ int32_t cenote_renderer_set_guide(cenote_renderer* r, cenote_guide* g, float fra
 
 int32_t cenote_renderer_set_material_sort(cenote_renderer* r, uint32_t mode) {
     CN_CHECK(r, CENOTE_E_INVALID_ARGUMENT, "null renderer");
-    CN_CHECK(mode <= CENOTE_SORT_SECONDARY, CENOTE_E_INVALID_ARGUMENT, "unknown material-sort mode");
+    CN_CHECK(mode <= CENOTE_SORT_SECONDARY || mode == CENOTE_SORT_AUTO, CENOTE_E_INVALID_ARGUMENT, "unknown material-sort mode");
     r->material_sort = mode;
-    r->sort_chosen = true;
     return CENOTE_OK;
 }
 
@@ -922,7 +921,8 @@ static uint32_t trav_variant_of(uint32_t block, uint32_t stack) {
 
 int32_t cenote_renderer_set_tuning(cenote_renderer* r, const cenote_tuning* t) {
     CN_CHECK(r && t, CENOTE_E_INVALID_ARGUMENT, "null argument");
-    CN_CHECK(t->material_sort <= CENOTE_SORT_SECONDARY, CENOTE_E_INVALID_ARGUMENT, "unknown material-sort mode");
+    CN_CHECK(t->material_sort <= CENOTE_SORT_SECONDARY || t->material_sort == CENOTE_SORT_AUTO,
+             CENOTE_E_INVALID_ARGUMENT, "unknown material-sort mode");
     CN_CHECK(t->refill_idle <= 32, CENOTE_E_INVALID_ARGUMENT, "refill threshold above a warp");
     CN_CHECK(t->top_nodes <= TOP_NODES_MAX, CENOTE_E_INVALID_ARGUMENT, "more top-level nodes than shared memory holds");
     CN_CHECK(t->l2_window <= 1, CENOTE_E_INVALID_ARGUMENT, "l2_window is 0 or 1");
@@ -933,7 +933,6 @@ int32_t cenote_renderer_set_tuning(cenote_renderer* r, const cenote_tuning* t) {
              "stack_depth is 16 or 32");
     CN_CHECK(t->sort_by_location <= 1, CENOTE_E_INVALID_ARGUMENT, "sort_by_location is 0 or 1");
     r->material_sort = t->material_sort;
-    r->sort_chosen = true;
     r->samples_per_wave = t->samples_per_wave;
     r->refill_idle = t->refill_idle;
     r->top_nodes = t->top_nodes;
@@ -1186,7 +1185,8 @@ int32_t cenote_renderer_autotune(cenote_renderer* r, cenote_scene* scene, uint32
     while (probe > 2 && pixels * probe > (uint64_t(1) << 27)) probe /= 2;
     const uint32_t saved_profiling = r->profiling;
     r->profiling = 0;
-    cenote_tuning best{r->material_sort,
+    // The tuned mode is one of the three that hold for every wave.
+    cenote_tuning best{r->material_sort == CENOTE_SORT_AUTO ? CENOTE_SORT_ALL : r->material_sort,
                        r->samples_per_wave,
                        r->refill_idle,
                        r->top_nodes,
@@ -1198,7 +1198,6 @@ int32_t cenote_renderer_autotune(cenote_renderer* r, cenote_scene* scene, uint32
                        r->sort_by_location};
     auto apply = [&](const cenote_tuning& t) {
         r->material_sort = t.material_sort;
-        r->sort_chosen = true;
         r->samples_per_wave = t.samples_per_wave;
         r->refill_idle = t.refill_idle;
         r->top_nodes = t.top_nodes;

@@ -192,11 +192,7 @@ struct cenote_renderer {
     std::vector<cudaEvent_t> events;
     PathPool pool{};
     DeviceBuffer ray, flux, hit, ps, q0, q1, shadows, shadow_queue, counters, tally, scratch;
-    // Material sort before shading: CENOTE_SORT_NONE, _ALL or _SECONDARY
-    // (every bounce by default: 1.1x on the material chart, 1.6x on the
-    // textured 2 M-triangle terrain, measured on a B200).
-    uint32_t material_sort = 1;
-    bool sort_chosen = false;  // set by the caller or the autotuner: then it holds for every wave
+    uint32_t material_sort = CENOTE_SORT_AUTO;  // CENOTE_SORT_*: see sort_mode
     uint32_t refill_idle = 0;  // 0: the kernels' default
     uint32_t top_nodes = 0;    // BVH nodes staged in shared memory by the traversal kernels
     uint32_t l2_window = 0;    // mark the BVH nodes persisting in L2 during this renderer's waves
@@ -253,24 +249,35 @@ struct cenote_renderer {
     }
 
     // The sort mode of a wave of `paths` camera paths (0: known on the device
-    // only). Unless a mode was chosen, waves whose bounces shade no faster in
-    // material order skip it, unless a guide trains on their records (which
-    // arrive in shading order); films are the same bits either way where the
-    // scene has no layered materials (with them, the sorted bounces split
-    // between two builds of the shading kernel). Measured device ms, sorted /
-    // unsorted: one closure class, 1 M paths, 36 to 20,412 triangles 1.58 /
-    // 1.43 to 2.87 / 2.67, 7.4 M paths 6.04 / 5.30 to 10.3 / 9.2; the chart at
-    // 0.23 M paths 1.00 / 0.91, at 0.92 M 1.69 / 1.75, at 16.6 M 16.7 / 19.4;
-    // the textured scene at 0.23 M 0.36 / 0.33, at 0.92 M 0.72 / 1.01.
+    // only). A chosen mode holds for every wave. Without one every bounce sorts
+    // (1.1x on the material chart, 1.6x on the textured terrain) but in the
+    // waves whose bounces shade no faster in material order, unless a guide
+    // trains on their records (which arrive in shading order); films are the
+    // same bits either way where the scene has no layered materials (with
+    // them, the sorted bounces split between two builds of the shading
+    // kernel).
+    //
+    // By paths: the sort's launches cost a bounce about 10 us, its order saves
+    // in proportion to the paths. Device ms unsorted / sorted of one-sample
+    // frames, the chart: 60 k paths 0.61 / 0.72, 230 k 0.83 / 0.95, 300 k 0.90 /
+    // 1.01, 600 k 1.19 / 1.27, 920 k 1.57 / 1.58, 1.4 M 2.08 / 2.01; the textured
+    // scene: 60 k 0.26 / 0.29, 230 k 0.34 / 0.36, 300 k 0.38 / 0.39, 450 k 0.475 /
+    // 0.467, 600 k 0.60 / 0.54, 1.4 M 1.30 / 0.96. The line lies below the first
+    // crossing, where no measured scene gains by sorting.
+    //
+    // By scene: one closure class, 36 to 20,412 triangles, sorted / unsorted
+    // 1.58 / 1.43 to 2.87 / 2.67 at 1 M paths, 6.04 / 5.30 to 10.3 / 9.2 at 7.4 M.
     static constexpr uint32_t SORT_MIN_PATHS = 1u << 18;
     static constexpr uint32_t UNIFORM_MAX_TRIANGLES = 1u << 15;
     uint32_t sort_mode(const cenote_scene* sc, uint32_t paths) const {
-        if (sort_chosen || sc->ds.has_layers || (guide && guide_steps > 0)) return material_sort;
+        if (material_sort != CENOTE_SORT_AUTO) return material_sort;
+        if (sc->ds.has_layers || (guide && guide_steps > 0)) return CENOTE_SORT_ALL;
         if (sc->uniform_shading || (paths != 0 && paths < SORT_MIN_PATHS)) return CENOTE_SORT_NONE;
-        return material_sort;
+        return CENOTE_SORT_ALL;
     }
 
-    // Free the pool and every lane sized by a wave (not the one-shot image); the next wave allocates anew.
+    // Free the pool and every lane sized by a wave (not the one-shot image);
+    // the next wave allocates anew.
     void release_pool() {
         pool_cap = aov_cap = g_cap = 0;
         for (DeviceBuffer* b : {&ray, &flux, &hit, &ps, &q0, &q1, &shadows, &shadow_queue, &sort_order, &sort_keys,

@@ -287,14 +287,15 @@ int32_t cenote_renderer_stats(cenote_renderer* r, cenote_stats* out);
 #define CENOTE_SORT_NONE 0u
 #define CENOTE_SORT_ALL 1u
 #define CENOTE_SORT_SECONDARY 2u /* every bounce but the camera rays' */
-/* A new renderer sorts every bounce (CENOTE_SORT_ALL) of the waves that gain
- * by it: small ones and scenes of one kind of material skip the sort, with the
- * same film. A mode set here holds for every wave. */
+/* A new renderer's: every bounce of the waves that gain by it; small ones and
+ * scenes of one kind of material skip the sort, with the same film. Any other
+ * mode holds for every wave. */
+#define CENOTE_SORT_AUTO 0xffffffffu
 int32_t cenote_renderer_set_material_sort(cenote_renderer* r, uint32_t mode);
 /* The per-scene launch knobs. None changes a result: every setting renders
  * the same film bit for bit. */
 typedef struct cenote_tuning {
-    uint32_t material_sort;    /* CENOTE_SORT_* */
+    uint32_t material_sort;    /* CENOTE_SORT_* (a new renderer reports CENOTE_SORT_AUTO) */
     uint32_t samples_per_wave; /* samples of every pixel one wave carries (0 = automatic); sets the queue capacity */
     uint32_t refill_idle;      /* idle lanes (1..32) before a traversal warp takes new rays (0 = default 8) */
     uint32_t top_nodes;        /* BVH top-level nodes staged in shared memory per traversal block (0..320) */

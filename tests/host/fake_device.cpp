@@ -20,7 +20,7 @@ std::mutex mu;
 std::map<uint64_t, uint64_t> live;  // address -> bytes
 uint64_t next_address = 1ull << 40, live_bytes = 0, limit = 180ull << 30, refused_size = ~0ull;
 uint64_t meminfo_calls = 0, bad_launches = 0, window_free_shadows = 0, windowed_walks = 0;
-uint64_t bytes_at_leaves = 0, waves = 0, largest_wave = 0;
+uint64_t bytes_at_leaves = 0, sorts = 0, waves = 0, largest_wave = 0;
 int refuse_after = -1;  // this many more allocations succeed, then one is refused
 cudaError_t last_error = cudaSuccess;
 bool hang = false;
@@ -61,6 +61,7 @@ uint64_t fake_open_windows() {
     return n;
 }
 uint64_t fake_bytes_at_leaves() { return bytes_at_leaves; }
+uint64_t fake_sorts() { return sorts; }
 uint64_t fake_waves() { return waves; }
 uint64_t fake_largest_wave() { return largest_wave; }
 double fake_clock_ms() { return std::chrono::duration<double, std::milli>(clock_offset).count(); }
@@ -198,6 +199,7 @@ void launch_shadow(const DeviceScene&, const PathPool&, uint32_t, const LaunchSh
     else window_free_shadows++;
 }
 void launch_material_sort(const PathPool& p, uint32_t, uint32_t n0, const LaunchShape&, cudaStream_t) {
+    sorts++;
     check(holds(p.order, 4ull * n0) && holds(p.sort_keys, 4ull * n0) && holds(p.sort_bins, 4 * SORT_BINS));
 }
 void launch_accumulate(const PathPool&, const FilmTargets& f, uint32_t base, uint32_t count, uint32_t, uint32_t, bool,

@@ -282,11 +282,49 @@ def waits_keep_their_bounds(lib):
         assert bound <= (lib.fake_clock_ms() - before) / 1e3 <= bound + 1
 
 
+def the_sort_stays_automatic_until_a_mode_is_chosen(lib):
+    """Reading a renderer's knobs and writing them back, or setting another knob,
+    leaves the automatic sort on; a mode holds for every wave."""
+    from cenote_b200 import SORT_ALL, SORT_AUTO, SORT_NONE, SORT_SECONDARY, CenoteError, Context, Film, Renderer
+
+    ctx = Context(0)
+    scene, film = small_scene(ctx), Film(ctx, 32, 32)  # a wave that skips the sort
+
+    def sorts(r):
+        before = lib.fake_sorts()
+        r.accumulate(scene, film, 1)
+        return lib.fake_sorts() - before
+
+    r = Renderer(ctx, 3)
+    assert sorts(r) == 0
+    t = r.tuning()
+    assert t["material_sort"] == SORT_AUTO
+    t.pop("ms_per_sample")
+    r.set_tuning(**t)
+    assert r.tuning()["material_sort"] == SORT_AUTO and sorts(r) == 0
+    r.set_tuning(**{**t, "refill_idle": 8})
+    assert sorts(r) == 0
+    for mode, n in ((SORT_ALL, 3), (SORT_SECONDARY, 2), (SORT_NONE, 0)):
+        r.set_material_sort(mode)
+        assert r.tuning()["material_sort"] == mode and sorts(r) == n
+        r.set_tuning(**{**t, "material_sort": mode, "refill_idle": 4})
+        assert sorts(r) == n
+    for bad in (3, 0xFFFFFFFE):
+        with pytest.raises(CenoteError):
+            r.set_material_sort(bad)
+        with pytest.raises(CenoteError):
+            r.set_tuning(bad)
+    r.set_material_sort(SORT_AUTO)
+    assert sorts(r) == 0
+    assert r.autotune(scene, 32, 32)["material_sort"] in (SORT_NONE, SORT_ALL, SORT_SECONDARY)
+
+
 SCENARIOS = {f.__name__: f for f in (a_refused_one_shot_image, a_refused_pool, refused_guide_lanes,
                                      a_refused_guide_batch, guide_lanes_fit_the_guided_wave,
                                      the_same_call_gets_the_same_wave, large_pools_are_given_back,
                                      a_refused_large_wave_is_a_plain_one, a_capacity_bounds_the_waves,
-                                     the_l2_window_covers_every_walk, waits_keep_their_bounds)}
+                                     the_l2_window_covers_every_walk, waits_keep_their_bounds,
+                                     the_sort_stays_automatic_until_a_mode_is_chosen)}
 
 
 @pytest.mark.parametrize("name", SCENARIOS)
