@@ -441,26 +441,7 @@ static int32_t create_scene(cenote_context* ctx, const cenote_object* objects, u
     cudaError_t err = cudaSuccess;
 
     std::vector<GeomRecord> geoms(object_count);
-    std::vector<Material> mats(object_count);
-    std::vector<BuildTri> tris;
-    std::vector<TriLight> tri_lights;
-    size_t total_tris = 0;
-    for (uint32_t i = 0; i < object_count; ++i) total_tris += objects[i].triangle_count;
-    tris.reserve(total_tris);
-    // Every mesh's vertices and indices end to end: one upload per stream, from
-    // which the device writes the triangles' attribute records.
-    std::vector<uint32_t> first_tri(size_t(object_count) + 1, 0);
-    std::vector<uint64_t> first_vertex(object_count, 0);
-    size_t total_vertices = 0;
-    for (uint32_t i = 0; i < object_count; ++i) total_vertices += objects[i].vertex_count;
-    CN_CHECK(total_tris < (1ull << 32), CENOTE_E_SCENE, "the scene's triangles exceed 32 bits");
-    std::vector<float> positions, normals, uvs;
-    std::vector<uint32_t> indices;
-    positions.reserve(3 * total_vertices);
-    normals.reserve(3 * total_vertices);
-    uvs.reserve(2 * total_vertices);
-    indices.reserve(3 * total_tris);
-    bool nonopaque = false, layered = false;
+    size_t total_tris = 0, total_vertices = 0;
     for (uint32_t i = 0; i < object_count; ++i) {
         const cenote_object& o = objects[i];
         CN_CHECK(o.positions && o.normals && o.uvs && o.indices && o.vertex_count > 0, CENOTE_E_INVALID_ARGUMENT,
@@ -474,6 +455,28 @@ static int32_t create_scene(cenote_context* ctx, const cenote_object* objects, u
         CN_CHECK(invert_affine(o.transform, g.w2o), CENOTE_E_INVALID_ARGUMENT,
                  "object " + std::to_string(i) + " transform is not invertible");
         g.light = LIGHT_NONE;
+        total_tris += o.triangle_count;
+        total_vertices += o.vertex_count;
+    }
+    CN_CHECK(total_tris < (1ull << 32), CENOTE_E_SCENE, "the scene's triangles exceed 32 bits");
+    std::vector<Material> mats(object_count);
+    std::vector<BuildTri> tris;
+    std::vector<TriLight> tri_lights;
+    tris.reserve(total_tris);
+    // Every mesh's vertices and indices end to end: one upload per stream, from
+    // which the device writes the triangles' attribute records.
+    std::vector<uint32_t> first_tri(size_t(object_count) + 1, 0);
+    std::vector<uint64_t> first_vertex(object_count, 0);
+    std::vector<float> positions, normals, uvs;
+    std::vector<uint32_t> indices;
+    positions.reserve(3 * total_vertices);
+    normals.reserve(3 * total_vertices);
+    uvs.reserve(2 * total_vertices);
+    indices.reserve(3 * total_tris);
+    bool nonopaque = false, layered = false;
+    for (uint32_t i = 0; i < object_count; ++i) {
+        const cenote_object& o = objects[i];
+        GeomRecord& g = geoms[i];
         first_vertex[i] = positions.size() / 3;
         first_tri[i + 1] = first_tri[i] + o.triangle_count;
         positions.insert(positions.end(), o.positions, o.positions + 3 * size_t(o.vertex_count));

@@ -319,12 +319,35 @@ def the_sort_stays_automatic_until_a_mode_is_chosen(lib):
     assert r.autotune(scene, 32, 32)["material_sort"] in (SORT_NONE, SORT_ALL, SORT_SECONDARY)
 
 
+def a_mesh_without_arrays_is_refused(lib):
+    """Counts of an object that is refused are not acted on."""
+    import ctypes
+
+    import cenote_b200
+    from cenote_b200 import CenoteError, Context, scenes
+
+    ctx = Context(0)
+    cam = cenote_b200._c_camera(scenes.cornell().camera)
+    texel = (ctypes.c_float * 4)()
+    env = cenote_b200.EnvironmentC(1, 1, ctypes.addressof(texel))
+    objects = (cenote_b200.Object * 4096)()
+    for o in objects:
+        o.vertex_count, o.triangle_count = 0xFFFFFFFF, 0
+        for slot in ("base_color", "specular_roughness", "metalness", "emission", "opacity", "normal"):
+            setattr(o.material, slot + "_texture", 0xFFFFFFFF)
+    h = ctypes.c_void_p()
+    with pytest.raises(CenoteError, match="object 0 lacks attributes"):
+        cenote_b200._check(lib.cenote_scene_create(ctx.handle, objects, len(objects), ctypes.byref(cam),
+                                                   ctypes.byref(env), None, 0, ctypes.byref(h)))
+
+
 SCENARIOS = {f.__name__: f for f in (a_refused_one_shot_image, a_refused_pool, refused_guide_lanes,
                                      a_refused_guide_batch, guide_lanes_fit_the_guided_wave,
                                      the_same_call_gets_the_same_wave, large_pools_are_given_back,
                                      a_refused_large_wave_is_a_plain_one, a_capacity_bounds_the_waves,
                                      the_l2_window_covers_every_walk, waits_keep_their_bounds,
-                                     the_sort_stays_automatic_until_a_mode_is_chosen)}
+                                     the_sort_stays_automatic_until_a_mode_is_chosen,
+                                     a_mesh_without_arrays_is_refused)}
 
 
 @pytest.mark.parametrize("name", SCENARIOS)
