@@ -394,6 +394,42 @@ cudaError_t upload_texture(const cenote_texture& t, cudaStream_t stream, cudaArr
     return e;
 }
 
+// One object's share of a stream of the concatenated meshes.
+struct Run {
+    const void* data;
+    size_t bytes;
+};
+
+// Upload every object's run (`of(object)`) end to end to `dst`: large runs from
+// the caller's memory, small ones gathered into one copy per 256 KB (a copy
+// call costs a few microseconds, however little it moves).
+template <class F>
+cudaError_t upload_runs(uint8_t* dst, const cenote_object* objects, uint32_t count, cudaStream_t s, F of) {
+    constexpr size_t LARGE = 64 << 10, BATCH = 256 << 10;
+    std::vector<uint8_t> batch;
+    cudaError_t e = cudaSuccess;
+    // From pageable memory the call returns once the bytes are staged.
+    auto copy = [&](const void* p, size_t n) {
+        if (n && e == cudaSuccess) e = cudaMemcpyAsync(dst, p, n, cudaMemcpyHostToDevice, s);
+        dst += n;
+    };
+    for (uint32_t i = 0; i < count && e == cudaSuccess; ++i) {
+        const Run r = of(objects[i]);
+        if (r.bytes >= LARGE || batch.size() + r.bytes > BATCH) {
+            copy(batch.data(), batch.size());
+            batch.clear();
+        }
+        if (r.bytes >= LARGE) {
+            copy(r.data, r.bytes);
+        } else {
+            const uint8_t* p = static_cast<const uint8_t*>(r.data);
+            batch.insert(batch.end(), p, p + r.bytes);
+        }
+    }
+    copy(batch.data(), batch.size());
+    return e;
+}
+
 }  // namespace
 
 extern "C" {
@@ -463,26 +499,18 @@ static int32_t create_scene(cenote_context* ctx, const cenote_object* objects, u
     std::vector<BuildTri> tris;
     std::vector<TriLight> tri_lights;
     tris.reserve(total_tris);
-    // Every mesh's vertices and indices end to end: one upload per stream, from
-    // which the device writes the triangles' attribute records.
+    // Every mesh's vertices and indices end to end on the device, from which it
+    // writes the triangles' attribute records.
     std::vector<uint32_t> first_tri(size_t(object_count) + 1, 0);
     std::vector<uint64_t> first_vertex(object_count, 0);
-    std::vector<float> positions, normals, uvs;
-    std::vector<uint32_t> indices;
-    positions.reserve(3 * total_vertices);
-    normals.reserve(3 * total_vertices);
-    uvs.reserve(2 * total_vertices);
-    indices.reserve(3 * total_tris);
+    for (uint32_t i = 0; i < object_count; ++i) {
+        first_tri[i + 1] = first_tri[i] + objects[i].triangle_count;
+        if (i) first_vertex[i] = first_vertex[i - 1] + objects[i - 1].vertex_count;
+    }
     bool nonopaque = false, layered = false;
     for (uint32_t i = 0; i < object_count; ++i) {
         const cenote_object& o = objects[i];
         GeomRecord& g = geoms[i];
-        first_vertex[i] = positions.size() / 3;
-        first_tri[i + 1] = first_tri[i] + o.triangle_count;
-        positions.insert(positions.end(), o.positions, o.positions + 3 * size_t(o.vertex_count));
-        normals.insert(normals.end(), o.normals, o.normals + 3 * size_t(o.vertex_count));
-        uvs.insert(uvs.end(), o.uvs, o.uvs + 2 * size_t(o.vertex_count));
-        indices.insert(indices.end(), o.indices, o.indices + 3 * size_t(o.triangle_count));
         mats[i] = o.material;
         V3 em = v3(o.material.emission);
         bool emissive = em.x != 0.0f || em.y != 0.0f || em.z != 0.0f;
@@ -529,27 +557,31 @@ static int32_t create_scene(cenote_context* ctx, const cenote_object* objects, u
     const uint32_t tri_count = uint32_t(tris.size());
     DeviceBuffer* battrs = sc->add(size_t(tri_count) * TRI_ATTRS * 16, &err);
     CN_CUDA(err);
-    DeviceBuffer mesh_stage;  // the six streams in one allocation (each one freed here waits for the device)
     {
-        const std::pair<const void*, size_t> streams[6] = {
-            {positions.data(), positions.size() * 4}, {normals.data(), normals.size() * 4},
-            {uvs.data(), uvs.size() * 4},             {indices.data(), indices.size() * 4},
-            {first_tri.data(), first_tri.size() * 4}, {first_vertex.data(), first_vertex.size() * 8}};
+        DeviceBuffer stage;  // the six streams in one allocation (each one freed here waits for the device)
         size_t at[7] = {0};
-        for (int k = 0; k < 6; ++k) at[k + 1] = at[k] + (streams[k].second + 255) / 256 * 256;
-        CN_CUDA(mesh_stage.alloc(at[6]));
-        uint8_t* stage = mesh_stage.as<uint8_t>();
-        for (int k = 0; k < 6; ++k)
-            if (streams[k].second)
-                CN_CUDA(cudaMemcpyAsync(stage + at[k], streams[k].first, streams[k].second, cudaMemcpyHostToDevice,
-                                        ctx->stream));
-        launch_attributes(reinterpret_cast<const float*>(stage + at[0]), reinterpret_cast<const float*>(stage + at[1]),
-                          reinterpret_cast<const float*>(stage + at[2]),
-                          reinterpret_cast<const uint32_t*>(stage + at[3]),
-                          reinterpret_cast<const uint32_t*>(stage + at[4]),
-                          reinterpret_cast<const uint64_t*>(stage + at[5]), object_count, tri_count,
+        const size_t bytes[6] = {12 * total_vertices,  12 * total_vertices,  8 * total_vertices,
+                                 12 * size_t(total_tris), first_tri.size() * 4, first_vertex.size() * 8};
+        for (int k = 0; k < 6; ++k) at[k + 1] = at[k] + (bytes[k] + 255) / 256 * 256;
+        CN_CUDA(stage.alloc(at[6]));
+        uint8_t* base = stage.as<uint8_t>();
+        CN_CUDA(upload_runs(base + at[0], objects, object_count, ctx->stream,
+                            [](const cenote_object& o) { return Run{o.positions, size_t(o.vertex_count) * 12}; }));
+        CN_CUDA(upload_runs(base + at[1], objects, object_count, ctx->stream,
+                            [](const cenote_object& o) { return Run{o.normals, size_t(o.vertex_count) * 12}; }));
+        CN_CUDA(upload_runs(base + at[2], objects, object_count, ctx->stream,
+                            [](const cenote_object& o) { return Run{o.uvs, size_t(o.vertex_count) * 8}; }));
+        CN_CUDA(upload_runs(base + at[3], objects, object_count, ctx->stream,
+                            [](const cenote_object& o) { return Run{o.indices, size_t(o.triangle_count) * 12}; }));
+        CN_CUDA(cudaMemcpyAsync(base + at[4], first_tri.data(), bytes[4], cudaMemcpyHostToDevice, ctx->stream));
+        CN_CUDA(cudaMemcpyAsync(base + at[5], first_vertex.data(), bytes[5], cudaMemcpyHostToDevice, ctx->stream));
+        launch_attributes(reinterpret_cast<const float*>(base + at[0]), reinterpret_cast<const float*>(base + at[1]),
+                          reinterpret_cast<const float*>(base + at[2]), reinterpret_cast<const uint32_t*>(base + at[3]),
+                          reinterpret_cast<const uint32_t*>(base + at[4]),
+                          reinterpret_cast<const uint64_t*>(base + at[5]), object_count, tri_count,
                           battrs->as<float4>(), ctx->stream);
         CN_CUDA(cudaGetLastError());
+        CN_CUDA(cudaStreamSynchronize(ctx->stream));
     }
     for (uint32_t i = 0; i < object_count; ++i) geoms[i].attrs = battrs->as<float4>() + size_t(first_tri[i]) * TRI_ATTRS;
     DeviceBuffer* bgeo = sc->add(geoms.size() * sizeof(GeomRecord), &err);

@@ -56,8 +56,10 @@ def main(scenarios: dict) -> None:
     cenote_b200.LIB_PATH = pathlib.Path(sys.argv[1])
     lib = cenote_b200.library()
     for name in ("live_bytes", "meminfo_calls", "bad_launches", "windowed_walks", "window_free_shadows",
-                 "open_windows", "bytes_at_leaves", "waves", "sorts", "largest_wave"):
+                 "open_windows", "late_stages", "waves", "sorts", "largest_wave"):
         getattr(lib, "fake_" + name).restype = ctypes.c_uint64
     lib.fake_limit.argtypes = lib.fake_refuse_above.argtypes = [ctypes.c_uint64]
+    lib.fake_stream.argtypes = [ctypes.c_int, ctypes.POINTER(ctypes.c_uint64)]
+    lib.fake_stream.restype = ctypes.c_void_p
     lib.fake_clock_ms.restype = ctypes.c_double
     scenarios[sys.argv[2]](lib)

@@ -11,6 +11,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <vector>
 
 #include "runtime.h"
 
@@ -20,11 +21,15 @@ std::mutex mu;
 std::map<uint64_t, uint64_t> live;  // address -> bytes
 uint64_t next_address = 1ull << 40, live_bytes = 0, limit = 180ull << 30, refused_size = ~0ull;
 uint64_t meminfo_calls = 0, bad_launches = 0, window_free_shadows = 0, windowed_walks = 0;
-uint64_t bytes_at_leaves = 0, sorts = 0, waves = 0, largest_wave = 0;
+uint64_t sorts = 0, waves = 0, largest_wave = 0;
 int refuse_after = -1;  // this many more allocations succeed, then one is refused
 cudaError_t last_error = cudaSuccess;
 bool hang = false;
 std::chrono::nanoseconds clock_offset{0};
+std::map<uint64_t, std::vector<uint8_t>> uploads;  // what was copied to a live address
+std::vector<uint8_t> streams[4];                   // the meshes' streams as the attribute kernel finds them
+const void* stage = nullptr;
+uint64_t late_stages = 0;
 std::map<cudaStream_t, uint64_t> windows;  // stream -> bytes of its access-policy window
 
 template <class T>
@@ -60,7 +65,11 @@ uint64_t fake_open_windows() {
     for (auto& w : windows) n += w.second != 0;
     return n;
 }
-uint64_t fake_bytes_at_leaves() { return bytes_at_leaves; }
+uint64_t fake_late_stages() { return late_stages; }
+const uint8_t* fake_stream(int k, uint64_t* bytes) {
+    *bytes = streams[k].size();
+    return streams[k].data();
+}
 uint64_t fake_sorts() { return sorts; }
 uint64_t fake_waves() { return waves; }
 uint64_t fake_largest_wave() { return largest_wave; }
@@ -87,6 +96,7 @@ cudaError_t cudaFree(void* p) {
     auto it = live.find(reinterpret_cast<uint64_t>(p));
     if (it == live.end()) return p ? last_error = cudaErrorInvalidValue : cudaSuccess;
     live_bytes -= it->second;
+    uploads.erase(uploads.lower_bound(it->first), uploads.lower_bound(it->first + it->second));
     live.erase(it);
     return cudaSuccess;
 }
@@ -94,6 +104,11 @@ cudaError_t cudaMemGetInfo(size_t* free_bytes, size_t* total) {
     meminfo_calls++;
     *free_bytes = limit - live_bytes;
     *total = limit;
+    return cudaSuccess;
+}
+cudaError_t cudaMemcpyAsync(void* dst, const void* src, size_t n, cudaMemcpyKind kind, cudaStream_t) {
+    const uint8_t* p = static_cast<const uint8_t*>(src);
+    if (kind == cudaMemcpyHostToDevice) uploads[reinterpret_cast<uint64_t>(dst)].assign(p, p + n);
     return cudaSuccess;
 }
 cudaError_t cudaMallocHost(void** p, size_t n) {
@@ -209,8 +224,23 @@ void launch_accumulate(const PathPool&, const FilmTargets& f, uint32_t base, uin
 void launch_copy_rad(const PathPool&, float4* out, uint32_t base, uint32_t count, uint32_t, cudaStream_t) {
     check(holds(out, 16 * (uint64_t(base) + count)));
 }
+void launch_attributes(const float* positions, const float* normals, const float* uvs, const uint32_t* indices,
+                       const uint32_t* first_tri, const uint64_t*, uint32_t, uint32_t n, float4* attrs, cudaStream_t) {
+    check(holds(attrs, 16ull * TRI_ATTRS * n));
+    stage = positions;
+    const void* begin[5] = {positions, normals, uvs, indices, first_tri};
+    for (int k = 0; k < 4; ++k) {
+        streams[k].clear();
+        uint64_t at = reinterpret_cast<uint64_t>(begin[k]);
+        for (auto it = uploads.find(at); it != uploads.end() && it->first == at &&
+                                         at < reinterpret_cast<uint64_t>(begin[k + 1]); it = uploads.find(at)) {
+            streams[k].insert(streams[k].end(), it->second.begin(), it->second.end());
+            at += it->second.size();
+        }
+    }
+}
 void launch_light_leaves(const float4*, uint32_t, const GeomRecord*, uint32_t*, cudaStream_t) {
-    bytes_at_leaves = live_bytes;
+    late_stages += holds(stage, 1);
 }
 
 namespace guide {

@@ -319,6 +319,40 @@ def the_sort_stays_automatic_until_a_mode_is_chosen(lib):
     assert r.autotune(scene, 32, 32)["material_sort"] in (SORT_NONE, SORT_ALL, SORT_SECONDARY)
 
 
+def meshes_are_staged_and_given_back(lib):
+    """Whatever the meshes' sizes, the device finds their streams end to end, and
+    the staging memory is gone before the tree is built."""
+    import ctypes
+
+    import numpy as np
+
+    from cenote_b200 import BVH_GPU_SAH, BVH_HOST_SAH, Context, Scene, scenes
+
+    ctx = Context(0)
+    rng = np.random.default_rng(3)
+
+    def mesh(vertices, triangles):
+        f = lambda n: rng.random((vertices, n), np.float32)
+        return scenes.Mesh(f(3), f(3), f(2), rng.integers(0, vertices, (triangles, 3)).astype(np.uint32))
+
+    # Runs below, at and above the sizes that are gathered (64 KB) and flushed (256 KB).
+    sizes = [(1, 1), (3, 0), (5461, 5461), (5462, 5462), (8191, 5461), (8192, 3), (3, 5462), (30000, 40000)]
+    sizes += [(5000, 5000)] * 9 + [(1, 0)]
+    for builder in (BVH_HOST_SAH, BVH_GPU_SAH):
+        ctx.set_bvh_builder(builder)
+        for order in (sizes, sizes[::-1], sizes[:1], sizes[1:2]):
+            spec = scenes.cornell()
+            meshes = [mesh(*n) for n in order]
+            spec.objects = [scenes.Object(m, scenes.rows(np.eye(4)), scenes.matte((0.5, 0.5, 0.5))) for m in meshes]
+            Scene(ctx, spec).close()
+            for k, name in enumerate(("positions", "normals", "uvs", "indices")):
+                n = ctypes.c_uint64()
+                data = lib.fake_stream(k, ctypes.byref(n))
+                want = b"".join(np.ascontiguousarray(getattr(m, name)).tobytes() for m in meshes)
+                assert ctypes.string_at(data, n.value) == want, (k, len(order))
+            assert lib.fake_late_stages() == 0
+
+
 def a_mesh_without_arrays_is_refused(lib):
     """Counts of an object that is refused are not acted on."""
     import ctypes
@@ -347,7 +381,7 @@ SCENARIOS = {f.__name__: f for f in (a_refused_one_shot_image, a_refused_pool, r
                                      a_refused_large_wave_is_a_plain_one, a_capacity_bounds_the_waves,
                                      the_l2_window_covers_every_walk, waits_keep_their_bounds,
                                      the_sort_stays_automatic_until_a_mode_is_chosen,
-                                     a_mesh_without_arrays_is_refused)}
+                                     meshes_are_staged_and_given_back, a_mesh_without_arrays_is_refused)}
 
 
 @pytest.mark.parametrize("name", SCENARIOS)
