@@ -1374,17 +1374,6 @@ void launch_shadow(const DeviceScene& scene, const PathPool& pool, uint32_t boun
     }
 }
 
-void launch_wave(const DeviceScene& scene, const PathPool& pool, const WaveParams& wp, const LaunchShape& ls,
-                 cudaStream_t stream) {
-    const uint32_t n0 = wp.pixel_count * wp.samples;
-    launch_wave_begin(pool, wp, ls, stream);
-    for (uint32_t b = 0; b < wp.max_bounces; ++b) {
-        launch_intersect(scene, pool, b, n0, ls, false, stream);
-        launch_shade(scene, pool, b, wp, n0, ls, stream);
-        launch_shadow(scene, pool, b, ls, false, stream);
-    }
-}
-
 void launch_accumulate(const PathPool& pool, const FilmTargets& film, uint32_t pixel_base, uint32_t pixel_count,
                        uint32_t tile_width, uint32_t samples, bool reset, cudaStream_t stream) {
     int grid = int((pixel_count + 255) / 256);

@@ -184,11 +184,9 @@ struct LaunchShape {
 
 LaunchShape launch_shape(int device);
 
-// One wave: raygen, then max_bounces × (intersect, shade, shadow). Path
-// radiance lands in pool.rad(path) with path = s · pixel_count + local pixel.
-// The stages are also exposed one by one so a caller can time them.
-void launch_wave(const DeviceScene& scene, const PathPool& pool, const WaveParams& wp, const LaunchShape& ls,
-                 cudaStream_t stream);
+// The stages of a wave: raygen (launch_wave_begin), then max_bounces ×
+// (intersect, shade, shadow). Path radiance lands in pool.rad(path) with path =
+// s · pixel_count + local pixel.
 void launch_wave_begin(const PathPool& pool, const WaveParams& wp, const LaunchShape& ls, cudaStream_t stream);
 // `count_visits` selects the instrumented traversal that tallies wide-node
 // visits and triangle tests into the counters (for the roofline's traffic).
