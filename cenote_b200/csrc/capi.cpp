@@ -1213,12 +1213,12 @@ int32_t cenote_renderer_autotune(cenote_renderer* r, cenote_scene* scene, uint32
     std::lock_guard<std::mutex> lock(r->ctx->mu);
     CN_CUDA(cudaSetDevice(r->ctx->device));
     const uint64_t pixels = uint64_t(width) * height;
-    // The automatic wave size (plan_waves), its half, and 2x, 4x and 8x,
-    // bounded by 64 M paths (about 16 GB of path state).
-    const uint32_t auto_spw = uint32_t(std::max<uint64_t>(1, std::min<uint64_t>((uint64_t(1) << 24) / pixels, 64)));
+    // The automatic wave size, half of the plain wave's (2^24 paths), and 2x, 4x
+    // and 8x, bounded by 2^26 paths (14.8 GB of path state) and 256 samples.
+    const uint32_t plain = uint32_t(std::max<uint64_t>(1, std::min<uint64_t>(cenote_renderer::PLAIN_WAVE / pixels, 64)));
     const uint32_t spw_cap = uint32_t(std::max<uint64_t>(1, std::min<uint64_t>((uint64_t(1) << 26) / pixels, 256)));
-    const uint32_t spws[5] = {0, std::max(1u, auto_spw / 2), std::min(spw_cap, auto_spw * 2),
-                              std::min(spw_cap, auto_spw * 4), std::min(spw_cap, auto_spw * 8)};
+    const uint32_t spws[5] = {0, std::max(1u, plain / 2), std::min(spw_cap, plain * 2), std::min(spw_cap, plain * 4),
+                              std::min(spw_cap, plain * 8)};
     // Probe length: two waves of the largest candidate, at most ~128 M samples.
     uint32_t probe = std::max(2u, 2 * spws[4]);
     while (probe > 2 && pixels * probe > (uint64_t(1) << 27)) probe /= 2;

@@ -169,7 +169,9 @@ inline void plane_t(float a, float b, const PlanePair& p, float& n, float& f) {
 // is lowered by 2^-21 s and the far one raised by 2^-20 s, so the test also
 // accepts whatever the plain test q · aid + aor with its far planes scaled by
 // 1.0000004 accepts: a walk visits the same nodes and now and then one more,
-// and commits the same hits. The slack is below 0.07 of a cell.
+// and commits the same hits. The far slack, the larger one, is a sixteenth of
+// a cell plus 2^-20 of the corner's distance along the ray (|aor|): under 0.07
+// of a cell within 8,000 cells of a node, a whole cell at a million.
 __device__ __forceinline__ PlanePair node_axis(float aid, float aor) {
     const float s = fmaf(fabsf(aid), PLANE_BIAS, fabsf(aor));
     const float c = fmaf(-PLANE_BIAS, aid, aor);

@@ -39,8 +39,8 @@ constexpr uint32_t TQ_FULL = 0xffffffffu;
 // measured no gain from it).
 constexpr uint32_t TQ_WAITING = 8;
 
-// One warp's queue in shared memory (1,792 bytes: a full SM of traversal
-// blocks keeps 56 KB, and the L1 cache, which holds the walks' stacks and the
+// One warp's queue in shared memory (1,920 bytes: a full SM of traversal
+// blocks keeps 60 KB, and the L1 cache, which holds the walks' stacks and the
 // nodes and triangles they revisit, most of its capacity). What a lane's ray
 // needs only in the triangle rounds lives here instead of in registers: ten
 // registers a lane, without which the node test spilled.
@@ -56,6 +56,7 @@ struct TriQueueSmem {
     // shadow query's target (leaf, instance, primitive, unused).
     uint4 best[32];
 };
+static_assert(sizeof(TriQueueSmem) == 1920, "1,920 bytes a warp");
 
 // What a walking lane keeps of its ray: the node test's inputs.
 struct WalkRay {

@@ -297,7 +297,7 @@ int32_t cenote_renderer_set_material_sort(cenote_renderer* r, uint32_t mode);
 typedef struct cenote_tuning {
     uint32_t material_sort;    /* CENOTE_SORT_* (a new renderer reports CENOTE_SORT_AUTO) */
     uint32_t samples_per_wave; /* samples of every pixel one wave carries (0 = automatic); sets the queue capacity */
-    uint32_t refill_idle;      /* idle lanes (1..32) before a traversal warp takes new rays (0 = default 8) */
+    uint32_t refill_idle;      /* idle lanes (1..32) before a traversal warp takes new rays (0 = default 12) */
     uint32_t top_nodes;        /* BVH top-level nodes staged in shared memory per traversal block (0..320) */
     uint32_t l2_window;        /* 1: the BVH nodes are a persisting L2 access-policy window during the waves */
     uint32_t per_lane_triangles; /* 1: each traversal lane tests its own triangles; 0: a warp shares its
