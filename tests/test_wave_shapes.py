@@ -55,3 +55,57 @@ def test_one_large_wave_is_the_small_waves(ctx):
     f.reset()
     guided.accumulate(scene, f, 17)
     assert guided.stats()["samples_per_wave"] == 16
+
+
+@pytest.mark.parametrize("name,w,h,sorts", [("chart", 511, 513, False), ("chart", 512, 512, True),
+                                            ("textured", 511, 513, False), ("textured", 512, 512, True),
+                                            ("cornell", 512, 512, False)])
+def test_the_automatic_sort_changes_no_film(ctx, name, w, h, sorts):
+    """On both sides of 2^18 paths, where the default starts to sort (a scene of
+    one closure class never does), its film is each chosen mode's."""
+    from cenote_b200 import SORT_ALL, SORT_NONE
+
+    spec = {"cornell": scenes.cornell, "chart": lambda: scenes.chart(env_size=(64, 32)),
+            "textured": lambda: scenes.textured(size=16)}[name]()
+    scene, out = Scene(ctx, spec), []
+    for mode in (None, SORT_ALL, SORT_NONE):
+        r, f = Renderer(ctx, 4, material_sort=mode), Film(ctx, w, h)
+        r.accumulate(scene, f, 1)
+        out.append((f.all_averages(), r.stats()["kernel_launches"]))
+    assert out[0][1] == out[1 if sorts else 2][1] and out[1][1] != out[2][1]
+    for other, _ in out[1:]:
+        for k, v in other.items():
+            assert np.array_equal(v, out[0][0][k], equal_nan=True), k
+
+
+def test_renderers_of_one_context_in_turn(ctx):
+    """Two renderers taking turns, one with the L2 window on and both with their
+    own side streams, draw the films they draw alone."""
+    spec = scenes.chart(env_size=(64, 32))
+    scene, other = Scene(ctx, spec), Scene(ctx, scenes.textured(size=16))
+
+    def make():
+        a, b = Renderer(ctx, 6), Renderer(ctx, 5)
+        a.set_tuning(1, l2_window=1)
+        return a, b
+
+    sizes = (200, 121), (97, 300)
+    alone = []
+    for k, s in enumerate((scene, other)):
+        r, f = make()[k], Film(ctx, *sizes[k])
+        for n in (1, 3, 2):
+            r.accumulate(s, f, n)
+        alone.append(f.all_averages())
+    plain = Film(ctx, *sizes[0])
+    Renderer(ctx, 6).accumulate(scene, plain, 6)
+    for k, v in plain.all_averages().items():
+        assert np.array_equal(v, alone[0][k], equal_nan=True), k
+    (a, b), (fa, fb) = make(), (Film(ctx, *sizes[0]), Film(ctx, *sizes[1]))
+    shot = b.render(scene, 50, 40, 2)
+    for n in (1, 3, 2):
+        a.accumulate(scene, fa, n)
+        b.accumulate(other, fb, n)
+        assert np.array_equal(b.render(scene, 50, 40, 2), shot)
+    for film, want in ((fa, alone[0]), (fb, alone[1])):
+        for k, v in film.all_averages().items():
+            assert np.array_equal(v, want[k], equal_nan=True), k
