@@ -1224,7 +1224,10 @@ int32_t cenote_renderer_autotune(cenote_renderer* r, cenote_scene* scene, uint32
     while (probe > 2 && pixels * probe > (uint64_t(1) << 27)) probe /= 2;
     const uint32_t saved_profiling = r->profiling;
     r->profiling = 0;
-    // The tuned mode is one of the three that hold for every wave.
+    // The tuned mode is one of the three that hold for every wave; a failed call
+    // that found nothing better leaves the automatic one.
+    const uint32_t sort_before = r->material_sort;
+    bool found = false;
     cenote_tuning best{r->material_sort == CENOTE_SORT_AUTO ? CENOTE_SORT_ALL : r->material_sort,
                        r->samples_per_wave,
                        r->refill_idle,
@@ -1293,12 +1296,16 @@ int32_t cenote_renderer_autotune(cenote_renderer* r, cenote_scene* scene, uint32
             if (rc == CENOTE_OK && ms < best_ms) {
                 best = t;
                 best_ms = ms;
+                found = true;
             }
         }
     }
     r->profiling = saved_profiling;
     apply(best);
-    if (rc != CENOTE_OK) return rc;
+    if (rc != CENOTE_OK) {
+        if (!found) r->material_sort = sort_before;
+        return rc;
+    }
     best.ms_per_sample = best_ms / float(probe);
     r->tuned_ms_per_sample = best.ms_per_sample;
     if (out) *out = best;

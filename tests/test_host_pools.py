@@ -316,6 +316,10 @@ def the_sort_stays_automatic_until_a_mode_is_chosen(lib):
             r.set_tuning(bad)
     r.set_material_sort(SORT_AUTO)
     assert sorts(r) == 0
+    before = r.tuning()
+    lib.fake_refuse_after(5)  # the film is there, the pool is not
+    refused(lambda: r.autotune(scene, 256, 256))
+    assert r.tuning() == before
     assert r.autotune(scene, 32, 32)["material_sort"] in (SORT_NONE, SORT_ALL, SORT_SECONDARY)
 
 
