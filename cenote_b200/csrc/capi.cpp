@@ -1141,7 +1141,7 @@ int32_t run_waves(cenote_renderer* r, cenote_scene* sc, uint32_t width, uint32_t
         if (e == cudaSuccess && r->guide) e = r->guide->ensure(cenote_renderer::GUIDE_BATCH);
         return e;
     };
-    cudaError_t e = allocating(ctx, allocate);
+    cudaError_t e = allocating(ctx, allocate, r);
     if (e == cudaErrorMemoryAllocation && plan.need > cenote_renderer::PLAIN_WAVE) {
         r->release_pool();  // the memory was there a moment ago: a plain wave then
         plan = plan_waves(r, pixels, count, oneshot != nullptr, cenote_renderer::PLAIN_WAVE);

@@ -62,14 +62,19 @@ int32_t copy_out(cenote_context* ctx, void* host, const void* device, size_t byt
     return wait_stream(ctx->stream, ctx->sync_ev, timeout_ms);
 }
 
-bool give_back_pools(cenote_context* ctx) {
+bool give_back_pools(cenote_context* ctx, const cenote_renderer* busy) {
     std::lock_guard<std::mutex> list(ctx->renderers_mu);
     bool any = false;
-    for (cenote_renderer* r : ctx->renderers)
+    for (cenote_renderer* r : ctx->renderers) {
         if (r->pool_cap > cenote_renderer::PLAIN_WAVE) {
             r->release_pool();
             any = true;
         }
+        if (r != busy && r->oneshot.ptr) {
+            r->oneshot.release();
+            any = true;
+        }
+    }
     return any;
 }
 

@@ -426,17 +426,18 @@ inline void release(cenote_context* ctx) {
 
 namespace cn {
 
-// Free the pools of the context's renderers that are larger than a plain wave's
-// (they were taken because memory was plentiful). True when any was. The
-// caller holds ctx->mu, so no wave of the context is in flight.
-bool give_back_pools(cenote_context* ctx);
+// Free what the context's renderers keep for their next call only because memory
+// was plentiful: pools larger than a plain wave's, and the one-shot images of
+// all but `busy`. True when there was any. The caller holds ctx->mu, so no wave
+// of the context is in flight.
+bool give_back_pools(cenote_context* ctx, const cenote_renderer* busy = nullptr);
 
-// Allocations under ctx->mu: refused, they are tried once more if large pools
+// Allocations under ctx->mu: refused, they are tried once more if anything
 // could be given back.
 template <class F>
-cudaError_t allocating(cenote_context* ctx, F allocations) {
+cudaError_t allocating(cenote_context* ctx, F allocations, const cenote_renderer* busy = nullptr) {
     const cudaError_t e = allocations();
-    return e == cudaErrorMemoryAllocation && give_back_pools(ctx) ? allocations() : e;
+    return e == cudaErrorMemoryAllocation && give_back_pools(ctx, busy) ? allocations() : e;
 }
 
 // The same for a call that makes a new object and leaves nothing behind when

@@ -200,6 +200,28 @@ def large_pools_are_given_back(lib):
         o.close()
 
 
+def one_shot_images_are_given_back(lib):
+    """An image kept for a renderer's next one-shot render makes room for others,
+    but not in that renderer's own call."""
+    from cenote_b200 import Context, Film, Renderer
+
+    ctx = Context(0)
+    scene, r, other = small_scene(ctx), Renderer(ctx, 2, capacity=1 << 14), Renderer(ctx, 2)
+    for call in (lambda: Film(ctx, 400, 400).close(), lambda: other.render(scene, 100, 100)):
+        lib.fake_limit(lib.fake_live_bytes() + (10 << 30))
+        r.render(scene, 2000, 2000)  # 64 MB kept
+        lib.fake_limit(lib.fake_live_bytes() + 1000)
+        call()
+        lib.fake_limit(lib.fake_live_bytes() + (1 << 30))
+        r.render(scene, 2000, 2000)
+        assert lib.fake_bad_launches() == 0
+    # A renderer's own image stays while room is made for its pool.
+    fresh = Renderer(ctx, 2)
+    lib.fake_refuse_after(1)
+    fresh.render(scene, 500, 400)
+    assert lib.fake_bad_launches() == 0
+
+
 def a_refused_large_wave_is_a_plain_one(lib):
     """Memory that the device reports free but does not give: the call runs in
     waves of 2^24 paths, then and later."""
@@ -386,7 +408,8 @@ def a_mesh_without_arrays_is_refused(lib):
 SCENARIOS = {f.__name__: f for f in (a_refused_one_shot_image, a_refused_pool, refused_guide_lanes,
                                      a_refused_guide_batch, guide_lanes_fit_the_guided_wave,
                                      the_same_call_gets_the_same_wave, large_pools_are_given_back,
-                                     a_refused_large_wave_is_a_plain_one, a_capacity_bounds_the_waves,
+                                     one_shot_images_are_given_back, a_refused_large_wave_is_a_plain_one,
+                                     a_capacity_bounds_the_waves,
                                      the_l2_window_covers_every_walk, waits_keep_their_bounds,
                                      the_sort_stays_automatic_until_a_mode_is_chosen,
                                      meshes_are_staged_and_given_back, a_mesh_without_arrays_is_refused)}
